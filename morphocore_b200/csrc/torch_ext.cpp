@@ -100,65 +100,90 @@ double fill_value(int64_t op, int64_t padding, double padding_value, bool single
     return op == MC_OP_DILATION ? -std::numeric_limits<double>::infinity() : std::numeric_limits<double>::infinity();
 }
 
+/// Whether a call with these inputs will be differentiated. Calls that will not be (inference, or inputs that need no
+/// gradient) skip the autograd function, which saves about 2 us of host time, and the winner index of MAX / MIN merges,
+/// whose only reader is the backward pass: on (8, 3, 128, 128) -> 16 channels the search for it took four fifths of the
+/// call (57 us with it).
+bool differentiated(std::initializer_list<const torch::Tensor*> inputs)
+{
+    if (!at::GradMode::is_enabled()) return false;
+    for (const torch::Tensor* t : inputs)
+        if (t->requires_grad()) return true;
+    return false;
+}
+
+/// One forward dilation / erosion and what its backward pass needs.
+struct MorphoCall
+{
+    mc_desc d;
+    torch::Tensor input4d, weight4d, sample_weight, indices, output;
+};
+
+MorphoCall run_morpho_forward(const torch::Tensor& input, const torch::Tensor& weight, int64_t op, int64_t merge, int64_t padding, double padding_value,
+                              bool save_indices, double noise_scale)
+{
+    TORCH_CHECK(noise_scale >= 0.0, "noise_scale must be non negative");
+    MorphoCall call;
+    call.input4d = input_to_4d(input);
+    call.weight4d = weight_to_4d(weight);
+    const bool identity = merge == MC_MERGE_IDENTITY;
+    TORCH_CHECK(call.input4d.size(1) == call.weight4d.size(1) || identity, "Input channels must match weight input channels");
+    require_cuda(input, "input");
+    require_cuda(weight, "weight");
+    TORCH_CHECK(input.device() == weight.device(), "input and weight must be on the same device");
+    TORCH_CHECK(input.scalar_type() == weight.scalar_type(), "input and weight must have the same dtype");
+    if (identity)
+    {
+        TORCH_CHECK(call.weight4d.size(0) == call.input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
+        TORCH_CHECK(call.weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1");
+    }
+    const c10::cuda::CUDAGuard device_guard(input.device());
+    call.input4d = call.input4d.contiguous();
+    call.weight4d = call.weight4d.contiguous();
+    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
+
+    mc_desc& d = call.d;
+    d = make_desc(input4d, weight4d, op, merge);
+    d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
+    d.fill = fill_value(op, padding, padding_value, d.dtype == MC_F32);
+
+    // One structuring element per batch element, drawn on the weight's device from its generator
+    // (csrc/cpp/morpho_op_wrap.hxx:55-64).
+    if (noise_scale > 0.0)
+    {
+        const torch::Tensor noise =
+            (torch::rand({input4d.size(0), weight4d.size(0), weight4d.size(1), weight4d.size(2), weight4d.size(3)}, weight4d.options()) * 2.0 - 1.0)
+            * noise_scale;
+        call.sample_weight = (weight4d.unsqueeze(0) + noise).contiguous();
+        d.weight_batch_stride = weight4d.numel();
+    }
+    const torch::Tensor& kernel_weight = call.sample_weight.defined() ? call.sample_weight : weight4d;
+
+    call.output = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    if (save_indices && (merge == MC_MERGE_MAX || merge == MC_MERGE_MIN))
+        call.indices = at::empty(call.output.sizes(), input4d.options().dtype(torch::kInt));
+
+    const TraceRange trace("morphocore::morpho_forward");
+    check_status(mc_morpho_forward(&d, input4d.data_ptr(), kernel_weight.data_ptr(), call.output.data_ptr(),
+                                   call.indices.defined() ? call.indices.data_ptr<int32_t>() : nullptr, at::cuda::getCurrentCUDAStream().stream()));
+    return call;
+}
+
 class MorphoFunction : public torch::autograd::Function<MorphoFunction>
 {
 public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, int64_t op, int64_t merge,
                                  int64_t padding, double padding_value, bool save_indices, double noise_scale)
     {
-        TORCH_CHECK(noise_scale >= 0.0, "noise_scale must be non negative");
-        const int64_t original_dims = input.dim();
-        torch::Tensor input4d = input_to_4d(input);
-        torch::Tensor weight4d = weight_to_4d(weight);
-        const bool identity = merge == MC_MERGE_IDENTITY;
-        TORCH_CHECK(input4d.size(1) == weight4d.size(1) || identity, "Input channels must match weight input channels");
-        require_cuda(input, "input");
-        require_cuda(weight, "weight");
-        TORCH_CHECK(input.device() == weight.device(), "input and weight must be on the same device");
-        TORCH_CHECK(input.scalar_type() == weight.scalar_type(), "input and weight must have the same dtype");
-        if (identity)
-        {
-            TORCH_CHECK(weight4d.size(0) == input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
-            TORCH_CHECK(weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1");
-        }
-        const c10::cuda::CUDAGuard device_guard(input.device());
-        input4d = input4d.contiguous();
-        weight4d = weight4d.contiguous();
-
-        mc_desc d = make_desc(input4d, weight4d, op, merge);
-        d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
-        d.fill = fill_value(op, padding, padding_value, d.dtype == MC_F32);
-
-        // One structuring element per batch element, drawn on the weight's device from its generator
-        // (csrc/cpp/morpho_op_wrap.hxx:55-64).
-        torch::Tensor sample_weight;
-        if (noise_scale > 0.0)
-        {
-            const torch::Tensor noise =
-                (torch::rand({input4d.size(0), weight4d.size(0), weight4d.size(1), weight4d.size(2), weight4d.size(3)}, weight4d.options()) * 2.0 - 1.0)
-                * noise_scale;
-            sample_weight = (weight4d.unsqueeze(0) + noise).contiguous();
-            d.weight_batch_stride = weight4d.numel();
-        }
-        const torch::Tensor& kernel_weight = sample_weight.defined() ? sample_weight : weight4d;
-
-        torch::Tensor output = torch::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
-        torch::Tensor indices;
-        if (save_indices && (merge == MC_MERGE_MAX || merge == MC_MERGE_MIN))
-            indices = torch::empty(output.sizes(), input4d.options().dtype(torch::kInt));
-
-        const TraceRange trace("morphocore::morpho_forward");
-        check_status(mc_morpho_forward(&d, input4d.data_ptr(), kernel_weight.data_ptr(), output.data_ptr(),
-                                       indices.defined() ? indices.data_ptr<int32_t>() : nullptr, at::cuda::getCurrentCUDAStream().stream()));
-
-        ctx->save_for_backward({input4d, weight4d, indices, sample_weight});
+        const MorphoCall call = run_morpho_forward(input, weight, op, merge, padding, padding_value, save_indices, noise_scale);
+        ctx->save_for_backward({call.input4d, call.weight4d, call.indices, call.sample_weight});
         ctx->saved_data["op"] = op;
         ctx->saved_data["merge"] = merge;
-        ctx->saved_data["pad_kind"] = static_cast<int64_t>(d.pad_kind);
-        ctx->saved_data["fill"] = d.fill;
-        ctx->saved_data["input_dims"] = original_dims;
+        ctx->saved_data["pad_kind"] = static_cast<int64_t>(call.d.pad_kind);
+        ctx->saved_data["fill"] = call.d.fill;
+        ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
-        return output_to_original(output, original_dims);
+        return output_to_original(call.output, input.dim());
     }
 
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad_outputs)
@@ -203,6 +228,56 @@ public:
     }
 };
 
+/// Both outputs of MorphoPairFunction and what its backward pass needs.
+struct MorphoPairCall
+{
+    torch::Tensor input4d, weight4d, flipped, out_dilation, out_erosion;
+};
+
+MorphoPairCall run_morpho_pair_forward(const torch::Tensor& input, const torch::Tensor& weight, int64_t merge, int64_t padding, double padding_value)
+{
+    MorphoPairCall call;
+    call.input4d = input_to_4d(input);
+    call.weight4d = weight_to_4d(weight);
+    const bool identity = merge == MC_MERGE_IDENTITY;
+    TORCH_CHECK(call.input4d.size(1) == call.weight4d.size(1) || identity, "Input channels must match weight input channels");
+    require_cuda(input, "input");
+    require_cuda(weight, "weight");
+    TORCH_CHECK(input.device() == weight.device(), "input and weight must be on the same device");
+    TORCH_CHECK(input.scalar_type() == weight.scalar_type(), "input and weight must have the same dtype");
+    if (identity)
+    {
+        TORCH_CHECK(call.weight4d.size(0) == call.input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
+        TORCH_CHECK(call.weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1");
+    }
+    const c10::cuda::CUDAGuard device_guard(input.device());
+    call.input4d = call.input4d.contiguous();
+    call.weight4d = call.weight4d.contiguous();
+    call.flipped = call.weight4d.flip({2, 3}).contiguous();
+    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
+
+    mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
+    d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
+    d.fill = fill_value(MC_OP_DILATION, padding, padding_value, d.dtype == MC_F32);
+    call.out_dilation = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    call.out_erosion = at::empty_like(call.out_dilation);
+    void* const dilation_out = call.out_dilation.data_ptr();
+    void* const erosion_out = call.out_erosion.data_ptr();
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    const TraceRange trace("morphocore::morpho_pair_forward");
+    const int rc = mc_morpho_pair_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), dilation_out, erosion_out, stream);
+    if (rc == MC_ERR_UNSUPPORTED)
+    {
+        check_status(mc_morpho_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), dilation_out, nullptr, stream));
+        mc_desc e = d;
+        e.op = MC_OP_EROSION;
+        e.fill = fill_value(MC_OP_EROSION, padding, padding_value, d.dtype == MC_F32);
+        check_status(mc_morpho_forward(&e, input4d.data_ptr(), call.flipped.data_ptr(), erosion_out, nullptr, stream));
+    }
+    else check_status(rc);
+    return call;
+}
+
 /// dilation(x, w) and erosion(x, w) of the SAME input and structuring element, the two halves of the reference's
 /// sigma_layer (morphocore/functional/sigma_layer.py:73-83). The forward pass is one fused kernel where
 /// mc_morpho_pair_forward covers the case and two mc_morpho_forward calls otherwise; the backward pass is the two
@@ -215,51 +290,14 @@ public:
     static torch::autograd::tensor_list forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, int64_t merge,
                                                 int64_t padding, double padding_value)
     {
-        const int64_t original_dims = input.dim();
-        torch::Tensor input4d = input_to_4d(input);
-        torch::Tensor weight4d = weight_to_4d(weight);
-        const bool identity = merge == MC_MERGE_IDENTITY;
-        TORCH_CHECK(input4d.size(1) == weight4d.size(1) || identity, "Input channels must match weight input channels");
-        require_cuda(input, "input");
-        require_cuda(weight, "weight");
-        TORCH_CHECK(input.device() == weight.device(), "input and weight must be on the same device");
-        TORCH_CHECK(input.scalar_type() == weight.scalar_type(), "input and weight must have the same dtype");
-        if (identity)
-        {
-            TORCH_CHECK(weight4d.size(0) == input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
-            TORCH_CHECK(weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1");
-        }
-        const c10::cuda::CUDAGuard device_guard(input.device());
-        input4d = input4d.contiguous();
-        weight4d = weight4d.contiguous();
-        const torch::Tensor flipped = weight4d.flip({2, 3}).contiguous();
-
-        mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
-        d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
-        d.fill = fill_value(MC_OP_DILATION, padding, padding_value, d.dtype == MC_F32);
-        torch::Tensor out_dilation = torch::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
-        torch::Tensor out_erosion = torch::empty_like(out_dilation);
-        const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-        {
-            const TraceRange trace("morphocore::morpho_pair_forward");
-            const int rc = mc_morpho_pair_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), out_dilation.data_ptr(), out_erosion.data_ptr(), stream);
-            if (rc == MC_ERR_UNSUPPORTED)
-            {
-                check_status(mc_morpho_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), out_dilation.data_ptr(), nullptr, stream));
-                mc_desc e = d;
-                e.op = MC_OP_EROSION;
-                e.fill = fill_value(MC_OP_EROSION, padding, padding_value, d.dtype == MC_F32);
-                check_status(mc_morpho_forward(&e, input4d.data_ptr(), flipped.data_ptr(), out_erosion.data_ptr(), nullptr, stream));
-            }
-            else check_status(rc);
-        }
-        ctx->save_for_backward({input4d, weight4d, flipped});
+        const MorphoPairCall call = run_morpho_pair_forward(input, weight, merge, padding, padding_value);
+        ctx->save_for_backward({call.input4d, call.weight4d, call.flipped});
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["padding"] = padding;
         ctx->saved_data["padding_value"] = padding_value;
-        ctx->saved_data["input_dims"] = original_dims;
+        ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
-        return {output_to_original(out_dilation, original_dims), output_to_original(out_erosion, original_dims)};
+        return {output_to_original(call.out_dilation, input.dim()), output_to_original(call.out_erosion, input.dim())};
     }
 
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad_outputs)
@@ -319,49 +357,60 @@ torch::Tensor pair_alphas(const torch::Tensor& alpha, int64_t merge, int64_t out
     return alpha.numel() == pairs ? alpha.contiguous() : alpha.reshape({1}).expand({pairs}).contiguous();
 }
 
+/// One forward smorph and what its backward pass needs.
+struct SmorphCall
+{
+    torch::Tensor input4d, weight4d, output;
+};
+
+SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, int64_t merge)
+{
+    SmorphCall call;
+    call.input4d = input_to_4d(input);
+    call.weight4d = weight_to_4d(weight);
+    require_cuda(input, "input");
+    require_cuda(weight, "weight");
+    require_cuda(alpha, "alpha");
+    TORCH_CHECK(weight.device() == input.device() && alpha.device() == input.device(),
+                "input, weight and alpha must be on the same device (input on ", input.device(), ", weight on ", weight.device(),
+                ", alpha on ", alpha.device(), ")");
+    TORCH_CHECK(input.scalar_type() == weight.scalar_type() && input.scalar_type() == alpha.scalar_type(),
+                "input, weight and alpha must have the same dtype");
+    if (merge == MC_MERGE_IDENTITY)
+    {
+        TORCH_CHECK(call.weight4d.size(0) == call.input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
+        TORCH_CHECK(call.weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1, got ", call.weight4d.size(1));
+    }
+    else
+    {
+        TORCH_CHECK(call.input4d.size(1) == call.weight4d.size(1), "Input channels must match weight input channels");
+    }
+    const c10::cuda::CUDAGuard device_guard(input.device());
+    call.input4d = call.input4d.contiguous();
+    call.weight4d = call.weight4d.contiguous();
+    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
+    const torch::Tensor alphas = pair_alphas(alpha, merge, weight4d.size(0), input4d.size(1));
+
+    const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
+    call.output = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    const TraceRange trace("morphocore::smorph_forward");
+    check_status(mc_smorph_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), call.output.data_ptr(),
+                                   at::cuda::getCurrentCUDAStream().stream()));
+    return call;
+}
+
 class SmorphFunction : public torch::autograd::Function<SmorphFunction>
 {
 public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, int64_t merge)
     {
-        const int64_t original_dims = input.dim();
-        torch::Tensor input4d = input_to_4d(input);
-        torch::Tensor weight4d = weight_to_4d(weight);
-        require_cuda(input, "input");
-        require_cuda(weight, "weight");
-        require_cuda(alpha, "alpha");
-        TORCH_CHECK(weight.device() == input.device() && alpha.device() == input.device(),
-                    "input, weight and alpha must be on the same device (input on ", input.device(), ", weight on ", weight.device(),
-                    ", alpha on ", alpha.device(), ")");
-        TORCH_CHECK(input.scalar_type() == weight.scalar_type() && input.scalar_type() == alpha.scalar_type(),
-                    "input, weight and alpha must have the same dtype");
-        const bool identity = merge == MC_MERGE_IDENTITY;
-        if (identity)
-        {
-            TORCH_CHECK(weight4d.size(0) == input4d.size(1), "Identity mode requires weight.shape[0] == input.shape[1]");
-            TORCH_CHECK(weight4d.size(1) == 1, "Identity mode requires weight.shape[1] == 1, got ", weight4d.size(1));
-        }
-        else
-        {
-            TORCH_CHECK(input4d.size(1) == weight4d.size(1), "Input channels must match weight input channels");
-        }
-        const c10::cuda::CUDAGuard device_guard(input.device());
-        input4d = input4d.contiguous();
-        weight4d = weight4d.contiguous();
-        const torch::Tensor alphas = pair_alphas(alpha, merge, weight4d.size(0), input4d.size(1));
-
-        const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
-        torch::Tensor output = torch::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
-        const TraceRange trace("morphocore::smorph_forward");
-        check_status(mc_smorph_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), output.data_ptr(),
-                                       at::cuda::getCurrentCUDAStream().stream()));
-
+        const SmorphCall call = run_smorph_forward(input, weight, alpha, merge);
         // The backward pass reads the 4-D output: the merge target of MAX and MIN.
-        ctx->save_for_backward({output, alpha, input4d, weight4d});
+        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d});
         ctx->saved_data["merge"] = merge;
-        ctx->saved_data["input_dims"] = original_dims;
+        ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
-        return output_to_original(output, original_dims);
+        return output_to_original(call.output, input.dim());
     }
 
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad_outputs)
@@ -402,6 +451,43 @@ public:
     }
 };
 
+/// One forward smorph with the smooth channel merge and what its backward pass needs.
+struct SmorphScmCall
+{
+    torch::Tensor input4d, weight4d, betas, output;
+};
+
+SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, const torch::Tensor& beta)
+{
+    SmorphScmCall call;
+    call.input4d = input_to_4d(input);
+    call.weight4d = weight_to_4d(weight);
+    require_cuda(input, "input");
+    require_cuda(weight, "weight");
+    require_cuda(alpha, "alpha");
+    require_cuda(beta, "beta");
+    TORCH_CHECK(weight.device() == input.device() && alpha.device() == input.device() && beta.device() == input.device(),
+                "input, weight, alpha and beta must be on the same device (input on ", input.device(), ", weight on ", weight.device(),
+                ", alpha on ", alpha.device(), ", beta on ", beta.device(), ")");
+    TORCH_CHECK(input.scalar_type() == weight.scalar_type() && input.scalar_type() == alpha.scalar_type() && input.scalar_type() == beta.scalar_type(),
+                "input, weight, alpha and beta must have the same dtype");
+    TORCH_CHECK(call.input4d.size(1) == call.weight4d.size(1), "Input channels must match weight input channels");
+    TORCH_CHECK(beta.numel() == call.weight4d.size(0), "Beta must have shape [out_channels]");
+    const c10::cuda::CUDAGuard device_guard(input.device());
+    call.input4d = call.input4d.contiguous();
+    call.weight4d = call.weight4d.contiguous();
+    call.betas = beta.contiguous();
+    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
+    const torch::Tensor alphas = pair_alphas(alpha, MC_MERGE_SMOOTH, weight4d.size(0), input4d.size(1));
+
+    const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, MC_MERGE_SMOOTH);
+    call.output = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    const TraceRange trace("morphocore::smorph_scm_forward");
+    check_status(mc_smorph_scm_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), call.betas.data_ptr(), call.output.data_ptr(),
+                                       at::cuda::getCurrentCUDAStream().stream()));
+    return call;
+}
+
 /// Smorph with the smooth channel merge, the autograd function of torch.ops.morphocore.smorph_scm
 /// (reference: csrc/cpp/smorph_scm.cpp:13-96). beta holds one value per output channel.
 class SmorphScmFunction : public torch::autograd::Function<SmorphScmFunction>
@@ -410,37 +496,12 @@ public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, torch::Tensor alpha,
                                  torch::Tensor beta)
     {
-        const int64_t original_dims = input.dim();
-        torch::Tensor input4d = input_to_4d(input);
-        torch::Tensor weight4d = weight_to_4d(weight);
-        require_cuda(input, "input");
-        require_cuda(weight, "weight");
-        require_cuda(alpha, "alpha");
-        require_cuda(beta, "beta");
-        TORCH_CHECK(weight.device() == input.device() && alpha.device() == input.device() && beta.device() == input.device(),
-                    "input, weight, alpha and beta must be on the same device (input on ", input.device(), ", weight on ", weight.device(),
-                    ", alpha on ", alpha.device(), ", beta on ", beta.device(), ")");
-        TORCH_CHECK(input.scalar_type() == weight.scalar_type() && input.scalar_type() == alpha.scalar_type()
-                        && input.scalar_type() == beta.scalar_type(),
-                    "input, weight, alpha and beta must have the same dtype");
-        TORCH_CHECK(input4d.size(1) == weight4d.size(1), "Input channels must match weight input channels");
-        TORCH_CHECK(beta.numel() == weight4d.size(0), "Beta must have shape [out_channels]");
-        const c10::cuda::CUDAGuard device_guard(input.device());
-        input4d = input4d.contiguous();
-        weight4d = weight4d.contiguous();
-        const torch::Tensor alphas = pair_alphas(alpha, MC_MERGE_SMOOTH, weight4d.size(0), input4d.size(1));
-        const torch::Tensor betas = beta.contiguous();
-
-        const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, MC_MERGE_SMOOTH);
-        torch::Tensor output = torch::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
-        const TraceRange trace("morphocore::smorph_scm_forward");
-        check_status(mc_smorph_scm_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), betas.data_ptr(), output.data_ptr(),
-                                           at::cuda::getCurrentCUDAStream().stream()));
+        const SmorphScmCall call = run_smorph_scm_forward(input, weight, alpha, beta);
         // The backward pass reads the 4-D output: the final value of the soft merge.
-        ctx->save_for_backward({output, alpha, betas, input4d, weight4d});
-        ctx->saved_data["input_dims"] = original_dims;
+        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d});
+        ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
-        return output_to_original(output, original_dims);
+        return output_to_original(call.output, input.dim());
     }
 
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grad_outputs)
@@ -505,14 +566,21 @@ torch::Tensor widen(const torch::Tensor& t, const torch::Tensor& like, const cha
     return t.to(torch::kFloat);
 }
 
+torch::Tensor morpho_call(const torch::Tensor& input, const torch::Tensor& weight, int64_t op, int64_t merge, int64_t padding, double padding_value,
+                          bool save_indices, double noise_scale)
+{
+    if (differentiated({&input, &weight})) return MorphoFunction::apply(input, weight, op, merge, padding, padding_value, save_indices, noise_scale);
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return output_to_original(run_morpho_forward(input, weight, op, merge, padding, padding_value, false, noise_scale).output, input.dim());
+}
+
 torch::Tensor dilation(torch::Tensor input, torch::Tensor weight, int64_t merge, int64_t padding, double padding_value, bool save_indices,
                        double noise_scale)
 {
     if (is_reduced(input))
         return dilation(input.to(torch::kFloat), widen(weight, input, "weight"), merge, padding, padding_value, save_indices, noise_scale)
             .to(input.scalar_type());
-    return MorphoFunction::apply(input, weight, static_cast<int64_t>(MC_OP_DILATION), checked_merge(merge), checked_padding(padding), padding_value,
-                                 save_indices, noise_scale);
+    return morpho_call(input, weight, MC_OP_DILATION, checked_merge(merge), checked_padding(padding), padding_value, save_indices, noise_scale);
 }
 
 torch::Tensor erosion(torch::Tensor input, torch::Tensor weight, int64_t merge, int64_t padding, double padding_value, bool save_indices,
@@ -521,8 +589,7 @@ torch::Tensor erosion(torch::Tensor input, torch::Tensor weight, int64_t merge, 
     if (is_reduced(input))
         return erosion(input.to(torch::kFloat), widen(weight, input, "weight"), merge, padding, padding_value, save_indices, noise_scale)
             .to(input.scalar_type());
-    return MorphoFunction::apply(input, weight, static_cast<int64_t>(MC_OP_EROSION), checked_merge(merge), checked_padding(padding), padding_value,
-                                 save_indices, noise_scale);
+    return morpho_call(input, weight, MC_OP_EROSION, checked_merge(merge), checked_padding(padding), padding_value, save_indices, noise_scale);
 }
 
 /// Extension (not an operator of the reference): both halves of sigma_layer at once. MAX / MIN merges that keep their
@@ -537,9 +604,15 @@ std::tuple<torch::Tensor, torch::Tensor> dilation_erosion(torch::Tensor input, t
     }
     merge = checked_merge(merge);
     padding = checked_padding(padding);
-    if (save_indices && (merge == MC_MERGE_MAX || merge == MC_MERGE_MIN))
+    if (save_indices && (merge == MC_MERGE_MAX || merge == MC_MERGE_MIN) && differentiated({&input, &weight}))
         return {dilation(input, weight, merge, padding, padding_value, true, 0.0),
                 erosion(input, weight.flip({-2, -1}), merge, padding, padding_value, true, 0.0)};
+    if (!differentiated({&input, &weight}))
+    {
+        const at::AutoDispatchBelowADInplaceOrView guard;
+        const MorphoPairCall call = run_morpho_pair_forward(input, weight, merge, padding, padding_value);
+        return {output_to_original(call.out_dilation, input.dim()), output_to_original(call.out_erosion, input.dim())};
+    }
     const auto out = MorphoPairFunction::apply(input, weight, merge, padding, padding_value);
     return {out[0], out[1]};
 }
@@ -549,7 +622,9 @@ torch::Tensor smorph(torch::Tensor input, torch::Tensor weight, torch::Tensor al
     TORCH_CHECK(merge >= 0 && merge <= MC_MERGE_IDENTITY && merge != MC_MERGE_SMOOTH, "Unsupported merge operation for smorph");
     if (is_reduced(input))
         return smorph(input.to(torch::kFloat), widen(weight, input, "weight"), widen(alpha, input, "alpha"), merge).to(input.scalar_type());
-    return SmorphFunction::apply(input, weight, alpha, merge);
+    if (differentiated({&input, &weight, &alpha})) return SmorphFunction::apply(input, weight, alpha, merge);
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return output_to_original(run_smorph_forward(input, weight, alpha, merge).output, input.dim());
 }
 
 torch::Tensor smorph_scm(torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, torch::Tensor beta)
@@ -557,7 +632,9 @@ torch::Tensor smorph_scm(torch::Tensor input, torch::Tensor weight, torch::Tenso
     if (is_reduced(input))
         return smorph_scm(input.to(torch::kFloat), widen(weight, input, "weight"), widen(alpha, input, "alpha"), widen(beta, input, "beta"))
             .to(input.scalar_type());
-    return SmorphScmFunction::apply(input, weight, alpha, beta);
+    if (differentiated({&input, &weight, &alpha, &beta})) return SmorphScmFunction::apply(input, weight, alpha, beta);
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return output_to_original(run_smorph_scm_forward(input, weight, alpha, beta).output, input.dim());
 }
 
 }  // namespace
