@@ -42,6 +42,13 @@ enum mc_merge { MC_MERGE_MAX = 0, MC_MERGE_MIN = 1, MC_MERGE_ADD = 2, MC_MERGE_A
  * CPP/morpho_padding_policy.hpp:23-33) or the clamped edge pixel. */
 enum mc_pad_kind { MC_PAD_FILL = 0, MC_PAD_REPLICATE = 1 };
 
+/* Bits of mc_desc.flags, dilation / erosion functions only.
+ * FLIPPED_WEIGHT: w is read, and gw written, with both kernel axes reversed: the operation works with w[kH-1-kh, kW-1-kw]
+ *   at tap (kh, kw). It is how the Python layer's erosion hands over the structuring element as the user holds it
+ *   (the reference flips a copy first, morphocore/functional/erosion.py:89).
+ * ACCUMULATE: the backward functions add to what gx and gw hold instead of overwriting them. */
+enum mc_flags { MC_FLAG_FLIPPED_WEIGHT = 1, MC_FLAG_ACCUMULATE = 2 };
+
 enum mc_dtype { MC_F32 = 0, MC_F64 = 1 };
 
 enum mc_status
@@ -63,7 +70,11 @@ typedef struct mc_desc
     int32_t merge;    /* mc_merge */
     int32_t pad_kind; /* mc_pad_kind; ignored by the smorph functions (out-of-image taps are excluded) */
     int32_t dtype;    /* mc_dtype */
-    int32_t reserved; /* must be 0 */
+    union
+    {
+        int32_t flags;    /* mc_flags, 0 for none */
+        int32_t reserved; /* the field's former name */
+    };
     double fill;      /* border value of MC_PAD_FILL */
     int64_t weight_batch_stride; /* elements between the structuring elements of two batch elements
                                     ([B, Co, Ci', kH, kW] weights of the noise path, CU/morpho_cuda_launch.cuh:36); 0 = shared */
@@ -91,7 +102,7 @@ size_t mc_morpho_backward_workspace_bytes(const mc_desc* desc, int have_idx);
 
 /* Backward dilation / erosion. Replaces morpho_backward_cuda<op, T> (CU/morpho_op.cuh:21-24,
  * CU/morpho_op.cu:102-177). gx [B,Ci,H,W] and gw (shape of the shared structuring element) are
- * overwritten (zeroed then accumulated). idx is the tensor written by mc_morpho_forward or NULL. */
+ * overwritten (zeroed then accumulated; only accumulated with MC_FLAG_ACCUMULATE). idx is the tensor written by mc_morpho_forward or NULL. */
 int mc_morpho_backward(const mc_desc* desc, const void* x, const void* w, const int32_t* idx, const void* gy, void* gx, void* gw,
                        void* workspace, size_t workspace_bytes, void* stream);
 
@@ -125,6 +136,16 @@ size_t mc_smorph_backward_workspace_bytes(const mc_desc* desc);
  * like alpha_pairs) are overwritten. */
 int mc_smorph_backward(const mc_desc* desc, const void* x, const void* w, const void* alpha_pairs, const void* y, const void* gy, void* gx,
                        void* gw, void* galpha_pairs, void* workspace, size_t workspace_bytes, void* stream);
+
+/* The re-parametrised structuring element of smorph, w~ = t ((1 - t) / 2 flip(w) + (1 + t) / 2 w) with t = tanh(alpha of
+ * the pair) (morphocore/functional/smorph.py:60-68, where it is a chain of tensor operations). w and w_tilde are
+ * [Co, Ci, kH, kW] ([Co, 1, kH, kW] for identity). Of desc, Co, Ci, kH, kW, merge and dtype are used. */
+int mc_smorph_reparametrise(const mc_desc* desc, const void* w, const void* alpha_pairs, void* w_tilde, void* stream);
+
+/* Its gradient: gw is overwritten from gw_tilde, and the part of the alpha gradient that flows through w~ is ADDED to
+ * galpha_pairs (which mc_smorph_backward has filled with the operator's own part). */
+int mc_smorph_reparametrise_backward(const mc_desc* desc, const void* w, const void* alpha_pairs, const void* gw_tilde, void* gw,
+                                     void* galpha_pairs, void* stream);
 
 /* Smorph with the smooth channel merge ("Smorph SCM"): the Ci soft extrema c_i of an output pixel are merged by a
  * second soft extremum, final = sum_i q_i c_i / sum_i q_i with q_i = exp(beta[o] (c_i - ref)), ref = max_i c_i for

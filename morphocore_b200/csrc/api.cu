@@ -245,6 +245,31 @@ int mc_smorph_backward(const mc_desc* desc, const void* x, const void* w, const 
                                    static_cast<double*>(galpha_pairs), workspace, s);
 }
 
+int mc_smorph_reparametrise(const mc_desc* desc, const void* w, const void* alpha_pairs, void* w_tilde, void* stream)
+{
+    const int rc = validate(desc, false, desc != nullptr && desc->merge == MC_MERGE_SMOOTH);
+    if (rc != MC_OK) return rc;
+    MC_REQUIRE(w); MC_REQUIRE(alpha_pairs); MC_REQUIRE(w_tilde);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (desc->dtype == MC_F32)
+        return smorph_reparametrise<float>(*desc, static_cast<const float*>(w), static_cast<const float*>(alpha_pairs), static_cast<float*>(w_tilde), s);
+    return smorph_reparametrise<double>(*desc, static_cast<const double*>(w), static_cast<const double*>(alpha_pairs), static_cast<double*>(w_tilde), s);
+}
+
+int mc_smorph_reparametrise_backward(const mc_desc* desc, const void* w, const void* alpha_pairs, const void* gw_tilde, void* gw, void* galpha_pairs,
+                                     void* stream)
+{
+    const int rc = validate(desc, false, desc != nullptr && desc->merge == MC_MERGE_SMOOTH);
+    if (rc != MC_OK) return rc;
+    MC_REQUIRE(w); MC_REQUIRE(alpha_pairs); MC_REQUIRE(gw_tilde); MC_REQUIRE(gw); MC_REQUIRE(galpha_pairs);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (desc->dtype == MC_F32)
+        return smorph_reparametrise_backward<float>(*desc, static_cast<const float*>(w), static_cast<const float*>(alpha_pairs),
+                                                    static_cast<const float*>(gw_tilde), static_cast<float*>(gw), static_cast<float*>(galpha_pairs), s);
+    return smorph_reparametrise_backward<double>(*desc, static_cast<const double*>(w), static_cast<const double*>(alpha_pairs),
+                                                 static_cast<const double*>(gw_tilde), static_cast<double*>(gw), static_cast<double*>(galpha_pairs), s);
+}
+
 int mc_smorph_scm_forward(const mc_desc* desc, const void* x, const void* w, const void* alpha_pairs, const void* beta, void* y, void* stream)
 {
     const int rc = validate(desc, false, true);

@@ -71,8 +71,11 @@ struct Geometry
     int64_t weight_batch_stride;
     bool replicate;
     bool identity;
+    bool flipped;      // the structuring element is stored with both kernel axes reversed (MC_FLAG_FLIPPED_WEIGHT)
 
     __host__ __device__ int taps() const { return kH * kW; }
+    /// Where tap k's weight (and its gradient) lies in the stored structuring element.
+    __host__ __device__ int stored_tap(int k) const { return flipped ? kH * kW - 1 - k : k; }
     __host__ __device__ int64_t plane() const { return static_cast<int64_t>(H) * W; }
     __host__ __device__ int window_elems() const { return win_rows * win_stride; }
     __host__ __device__ int halo_top() const { return kH - 1 - pH; }
@@ -94,6 +97,7 @@ inline Geometry make_geometry(const mc_desc& d, int elem_bytes)
     g.weight_batch_stride = d.weight_batch_stride;
     g.replicate = d.pad_kind == MC_PAD_REPLICATE;
     g.identity = d.merge == MC_MERGE_IDENTITY;
+    g.flipped = (d.flags & MC_FLAG_FLIPPED_WEIGHT) != 0;
     return g;
 }
 
@@ -333,5 +337,8 @@ template <typename T> int smorph_backward(const mc_desc& d, const T* x, const T*
 template <typename T> int smorph_scm_forward(const mc_desc& d, const T* x, const T* w, const T* alpha, const T* beta, T* y, cudaStream_t stream);
 template <typename T> int smorph_scm_backward(const mc_desc& d, const T* x, const T* w, const T* alpha, const T* beta, const T* y, const T* gy, T* gx,
                                               T* gw, T* galpha, T* gbeta, void* ws, cudaStream_t stream);
+
+template <typename T> int smorph_reparametrise(const mc_desc& d, const T* w, const T* alpha, T* out, cudaStream_t stream);
+template <typename T> int smorph_reparametrise_backward(const mc_desc& d, const T* w, const T* alpha, const T* grad, T* gw, T* galpha, cudaStream_t stream);
 
 }  // namespace mc

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(THREADS) morpho_backward_scatter_kernel(const 
         const int ih = h + g.pH - kh, iw = w + g.pW - kw;
         if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) atomic_add(gxb + ch * plane + static_cast<int64_t>(ih) * g.W + iw, grad);
         if (a.copies > 0) atomic_add(bins + (ch * taps + k) * a.copies + lane_copy, grad);
-        else atomic_add(gwo + ch * taps + k, a.sign * grad);
+        else atomic_add(gwo + ch * taps + g.stored_tap(k), a.sign * grad);
     };
 
     if (a.vec)
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(THREADS) morpho_backward_scatter_kernel(const 
     {
         T sum = T(0);
         for (int c = 0; c < a.copies; c++) sum += bins[e * a.copies + c];
-        if (sum != T(0)) atomic_add(gwo + e, a.sign * sum);
+        if (sum != T(0)) atomic_add(gwo + e / taps * taps + g.stored_tap(e % taps), a.sign * sum);
     }
 }
 
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_kernel(const
         {
             const int o = e % OB, k = e / OB;
             T v = T(0);
-            if (o0 + o < o_end) v = __ldg(wb + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + k);
+            if (o0 + o < o_end) v = __ldg(wb + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + g.stored_tap(k));
             sw[e] = IS_MIN ? -v : v;
         }
         __syncthreads();
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_kernel(const
                 sum += bins[e * a.copies + c];
                 bins[e * a.copies + c] = T(0);
             }
-            if (sum != T(0) && o0 + o < o_end) atomic_add(a.gw + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + k, a.sign * sum);
+            if (sum != T(0) && o0 + o < o_end) atomic_add(a.gw + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + g.stored_tap(k), a.sign * sum);
         }
     }
     __syncthreads();
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_identity_kernel(co
         const int c = c_begin + n;
         stage_window_async<STRIDE>(sx0 + (n & 1) * WINDOW, a.x + (static_cast<int64_t>(b) * g.Ci + c) * plane, g, tile_h0, tile_w0, a.fill,
                                    [](int col) { return Row::at(col); });
-        for (int e = threadIdx.x; e < TAPS; e += THREADS) cp_async_element(sw0 + (n & 1) * TAPS_PAD + e, wbase + static_cast<int64_t>(c) * TAPS + e);
+        for (int e = threadIdx.x; e < TAPS; e += THREADS) cp_async_element(sw0 + (n & 1) * TAPS_PAD + e, wbase + static_cast<int64_t>(c) * TAPS + g.stored_tap(e));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_identity_kernel(co
                 sum += bins[e * a.copies + c];
                 bins[e * a.copies + c] = T(0);
             }
-            if (sum != T(0)) atomic_add(a.gw + static_cast<int64_t>(ci) * TAPS + e, a.sign * sum);
+            if (sum != T(0)) atomic_add(a.gw + static_cast<int64_t>(ci) * TAPS + g.stored_tap(e), a.sign * sum);
         }
         // the next channel's first bin update comes after its own barrier above
     }

@@ -3,6 +3,7 @@
 
 #include "dispatch.cuh"
 #include "morpho_backward.cuh"
+#include "zero.cuh"
 
 namespace mc
 {
@@ -16,11 +17,10 @@ int morpho_backward<MC_T>(const mc_desc& d, const MC_T* x, const MC_T* w, const 
     const size_t taps = static_cast<size_t>(d.kH) * d.kW;
     const size_t wnumel = static_cast<size_t>(d.Co) * (d.merge == MC_MERGE_IDENTITY ? 1 : d.Ci) * taps;
     // Both gradients are sums that the kernels below build up with atomic adds: start from zero.
-    if (cudaMemsetAsync(gx, 0, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W, stream) != cudaSuccess
-        || cudaMemsetAsync(gw, 0, sizeof(T) * wnumel, stream) != cudaSuccess)
+    if ((d.flags & MC_FLAG_ACCUMULATE) == 0)
     {
-        set_last_error("cudaMemsetAsync: %s", cudaGetErrorString(cudaGetLastError()));
-        return MC_ERR_CUDA;
+        const int rc = zero_buffers({{gx, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W}, {gw, sizeof(T) * wnumel}}, stream);
+        if (rc != MC_OK) return rc;
     }
     if (d.merge == MC_MERGE_MAX || d.merge == MC_MERGE_MIN)
     {

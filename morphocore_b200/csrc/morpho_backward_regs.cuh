@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_regs_kernel(
         {
             const int kw = e % WROW, kh = (e / WROW) % KW, o = e / (WROW * KW);
             T v = T(0);
-            if (kw < KW) v = __ldg(wb + (static_cast<int64_t>(o_begin + o) * wci + wi) * TAPS + kh * KW + kw);
+            if (kw < KW) v = __ldg(wb + (static_cast<int64_t>(o_begin + o) * wci + wi) * TAPS + g.stored_tap(kh * KW + kw));
             sw[e] = IS_MIN ? -v : v;
         }
     }
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_regs_kernel(
     {
         const T sum = totals[e];
         const int o = o_begin + e / TAPS, k = e % TAPS;
-        if (sum != T(0)) atomic_add(a.gw + (static_cast<int64_t>(o) * wci + wi) * TAPS + k, a.sign * sum);
+        if (sum != T(0)) atomic_add(a.gw + (static_cast<int64_t>(o) * wci + wi) * TAPS + g.stored_tap(k), a.sign * sum);
     }
 
     // Sum the private footprints: window position (t, u), t = 2 ty + r, u = 4 tx + c, is image pixel

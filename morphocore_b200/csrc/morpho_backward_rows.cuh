@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_rows_kernel(
         {
             const int o = e % OB, k = e / OB;
             T v = T(0);
-            if (o0 + o < o_end) v = __ldg(wb + (static_cast<int64_t>(o0 + o) * wci + wi) * TAPS + k);
+            if (o0 + o < o_end) v = __ldg(wb + (static_cast<int64_t>(o0 + o) * wci + wi) * TAPS + g.stored_tap(k));
             sw[e] = IS_MIN ? -v : v;
         }
         __syncthreads();
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_rows_kernel(
     {
         const T sum = totals[e];
         const int o = o_begin + e / TAPS, k = e % TAPS;
-        if (sum != T(0)) atomic_add(a.gw + (static_cast<int64_t>(o) * wci + wi) * TAPS + k, a.sign * sum);
+        if (sum != T(0)) atomic_add(a.gw + (static_cast<int64_t>(o) * wci + wi) * TAPS + g.stored_tap(k), a.sign * sum);
     }
 
     T* gxp = a.gx + (static_cast<int64_t>(b) * g.Ci + ci) * plane;

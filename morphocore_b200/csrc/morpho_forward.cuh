@@ -253,7 +253,7 @@ __device__ __forceinline__ void stage_weights(T* __restrict__ sw, const T* __res
         if (o0 + o < g.Co)
         {
             const int wi = g.identity ? 0 : c0 + c;
-            v = __ldg(w + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + k);
+            v = __ldg(w + (static_cast<int64_t>(o0 + o) * wci + wi) * taps + g.stored_tap(k));
         }
         sw[e] = IS_MIN ? -v : v;
     }
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(THREADS) morpho_find_tap_kernel(const ForwardA
                 const T* row = xp + static_cast<int64_t>(h + g.pH - kh) * g.W + w + g.pW;
                 for (int kw = 0; kw < g.kW; kw++)
                 {
-                    const T wv = __ldg(wk + kh * g.kW + kw);
+                    const T wv = __ldg(wk + g.stored_tap(kh * g.kW + kw));
                     const T xv = __ldg(row - kw);
                     const T v = IS_MIN ? xv - wv : xv + wv;
                     if (strictly_better<IS_MIN>(v, best))
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(THREADS) morpho_find_tap_kernel(const ForwardA
                 for (int kw = 0; kw < g.kW; kw++)
                 {
                     const T xv = read_border(xp, g, h + g.pH - kh, w + g.pW - kw, a.fill);
-                    const T wv = __ldg(wk + kh * g.kW + kw);
+                    const T wv = __ldg(wk + g.stored_tap(kh * g.kW + kw));
                     const T v = IS_MIN ? xv - wv : xv + wv;
                     if (strictly_better<IS_MIN>(v, best))
                     {
@@ -595,7 +595,11 @@ __global__ void __launch_bounds__(FIND_TILE * FIND_TILE) morpho_find_tap_tiled_k
         for (int o = 0; o < g.Co; o++)
         {
             __syncthreads();   // windows landed (first pass); the previous output channel's structuring elements are no longer read
-            for (int e = threadIdx.x; e < cc * TAPS; e += NT) sw[e] = __ldg(wb + (static_cast<int64_t>(o) * g.Ci + c0) * TAPS + e);
+            for (int e = threadIdx.x; e < cc * TAPS; e += NT)
+            {
+                const int c = e / TAPS;
+                sw[e] = __ldg(wb + (static_cast<int64_t>(o) * g.Ci + c0 + c) * TAPS + g.stored_tap(e - c * TAPS));
+            }
             const int packed = next;
             if (live && o + 1 < g.Co) next = a.idx[at0 + static_cast<int64_t>(o + 1) * plane];
             __syncthreads();

@@ -3,6 +3,7 @@
 
 #include "dispatch.cuh"
 #include "smorph.cuh"
+#include "zero.cuh"
 
 namespace mc
 {
@@ -46,13 +47,9 @@ int smorph_backward<MC_T>(const mc_desc& d, const MC_T* x, const MC_T* w, const 
     const bool identity = d.merge == MC_MERGE_IDENTITY;
     const size_t wnumel = static_cast<size_t>(d.Co) * (identity ? 1 : d.Ci) * taps;
     const size_t anumel = identity ? d.Co : static_cast<size_t>(d.Co) * d.Ci;
-    if (cudaMemsetAsync(gx, 0, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W, stream) != cudaSuccess
-        || cudaMemsetAsync(gw, 0, sizeof(T) * wnumel, stream) != cudaSuccess
-        || cudaMemsetAsync(galpha, 0, sizeof(T) * anumel, stream) != cudaSuccess)
-    {
-        set_last_error("cudaMemsetAsync: %s", cudaGetErrorString(cudaGetLastError()));
-        return MC_ERR_CUDA;
-    }
+    const int zeroed =
+        zero_buffers({{gx, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W}, {gw, sizeof(T) * wnumel}, {galpha, sizeof(T) * anumel}}, stream);
+    if (zeroed != MC_OK) return zeroed;
     const T* counts = nullptr;
     if (d.merge == MC_MERGE_MAX || d.merge == MC_MERGE_MIN)
     {
@@ -99,14 +96,9 @@ int smorph_scm_backward<MC_T>(const mc_desc& d, const MC_T* x, const MC_T* w, co
 {
     using T = MC_T;
     const size_t taps = static_cast<size_t>(d.kH) * d.kW, pixels = static_cast<size_t>(d.B) * d.Co * d.H * d.W;
-    if (cudaMemsetAsync(gx, 0, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W, stream) != cudaSuccess
-        || cudaMemsetAsync(gw, 0, sizeof(T) * d.Co * d.Ci * taps, stream) != cudaSuccess
-        || cudaMemsetAsync(galpha, 0, sizeof(T) * d.Co * d.Ci, stream) != cudaSuccess
-        || cudaMemsetAsync(gbeta, 0, sizeof(T) * d.Co, stream) != cudaSuccess)
-    {
-        set_last_error("cudaMemsetAsync: %s", cudaGetErrorString(cudaGetLastError()));
-        return MC_ERR_CUDA;
-    }
+    const int zeroed = zero_buffers({{gx, sizeof(T) * static_cast<size_t>(d.B) * d.Ci * d.H * d.W}, {gw, sizeof(T) * d.Co * d.Ci * taps},
+                                     {galpha, sizeof(T) * d.Co * d.Ci}, {gbeta, sizeof(T) * d.Co}}, stream);
+    if (zeroed != MC_OK) return zeroed;
     // One more pass over every channel for the extremum and the sum of the channel weights of each output pixel.
     T* soft_ref = static_cast<T*>(ws);
     T* soft_inv = soft_ref + pixels;

@@ -120,7 +120,7 @@ struct MorphoCall
 };
 
 MorphoCall run_morpho_forward(const torch::Tensor& input, const torch::Tensor& weight, int64_t op, int64_t merge, int64_t padding, double padding_value,
-                              bool save_indices, double noise_scale)
+                              bool save_indices, double noise_scale, int64_t flags)
 {
     TORCH_CHECK(noise_scale >= 0.0, "noise_scale must be non negative");
     MorphoCall call;
@@ -146,6 +146,7 @@ MorphoCall run_morpho_forward(const torch::Tensor& input, const torch::Tensor& w
     d = make_desc(input4d, weight4d, op, merge);
     d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
     d.fill = fill_value(op, padding, padding_value, d.dtype == MC_F32);
+    d.flags = static_cast<int32_t>(flags);
 
     // One structuring element per batch element, drawn on the weight's device from its generator
     // (csrc/cpp/morpho_op_wrap.hxx:55-64).
@@ -173,14 +174,15 @@ class MorphoFunction : public torch::autograd::Function<MorphoFunction>
 {
 public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, int64_t op, int64_t merge,
-                                 int64_t padding, double padding_value, bool save_indices, double noise_scale)
+                                 int64_t padding, double padding_value, bool save_indices, double noise_scale, int64_t flags)
     {
-        const MorphoCall call = run_morpho_forward(input, weight, op, merge, padding, padding_value, save_indices, noise_scale);
+        const MorphoCall call = run_morpho_forward(input, weight, op, merge, padding, padding_value, save_indices, noise_scale, flags);
         ctx->save_for_backward({call.input4d, call.weight4d, call.indices, call.sample_weight});
         ctx->saved_data["op"] = op;
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["pad_kind"] = static_cast<int64_t>(call.d.pad_kind);
         ctx->saved_data["fill"] = call.d.fill;
+        ctx->saved_data["flags"] = flags;
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
         return output_to_original(call.output, input.dim());
@@ -206,6 +208,7 @@ public:
         mc_desc d = make_desc(input, weight, ctx->saved_data["op"].toInt(), ctx->saved_data["merge"].toInt());
         d.pad_kind = static_cast<int32_t>(ctx->saved_data["pad_kind"].toInt());
         d.fill = ctx->saved_data["fill"].toDouble();
+        d.flags = static_cast<int32_t>(ctx->saved_data["flags"].toInt());
         // The noisy weights chose the winning taps; grad_weight keeps the shared shape, summed over the batch.
         const torch::Tensor& kernel_weight = sample_weight.defined() ? sample_weight : weight;
         if (sample_weight.defined()) d.weight_batch_stride = weight.numel();
@@ -224,14 +227,14 @@ public:
 
         grad_input = output_to_original(grad_input, ctx->saved_data["input_dims"].toInt());
         if (ctx->saved_data["weight_dims"].toInt() == 2) grad_weight = grad_weight.squeeze(0).squeeze(0);
-        return {grad_input, grad_weight, torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor()};
+        return {grad_input, grad_weight, torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor(), torch::Tensor()};
     }
 };
 
 /// Both outputs of MorphoPairFunction and what its backward pass needs.
 struct MorphoPairCall
 {
-    torch::Tensor input4d, weight4d, flipped, out_dilation, out_erosion;
+    torch::Tensor input4d, weight4d, out_dilation, out_erosion;
 };
 
 MorphoPairCall run_morpho_pair_forward(const torch::Tensor& input, const torch::Tensor& weight, int64_t merge, int64_t padding, double padding_value)
@@ -253,7 +256,6 @@ MorphoPairCall run_morpho_pair_forward(const torch::Tensor& input, const torch::
     const c10::cuda::CUDAGuard device_guard(input.device());
     call.input4d = call.input4d.contiguous();
     call.weight4d = call.weight4d.contiguous();
-    call.flipped = call.weight4d.flip({2, 3}).contiguous();
     const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
 
     mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
@@ -271,8 +273,9 @@ MorphoPairCall run_morpho_pair_forward(const torch::Tensor& input, const torch::
         check_status(mc_morpho_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), dilation_out, nullptr, stream));
         mc_desc e = d;
         e.op = MC_OP_EROSION;
+        e.flags = MC_FLAG_FLIPPED_WEIGHT;
         e.fill = fill_value(MC_OP_EROSION, padding, padding_value, d.dtype == MC_F32);
-        check_status(mc_morpho_forward(&e, input4d.data_ptr(), call.flipped.data_ptr(), erosion_out, nullptr, stream));
+        check_status(mc_morpho_forward(&e, input4d.data_ptr(), weight4d.data_ptr(), erosion_out, nullptr, stream));
     }
     else check_status(rc);
     return call;
@@ -281,9 +284,8 @@ MorphoPairCall run_morpho_pair_forward(const torch::Tensor& input, const torch::
 /// dilation(x, w) and erosion(x, w) of the SAME input and structuring element, the two halves of the reference's
 /// sigma_layer (morphocore/functional/sigma_layer.py:73-83). The forward pass is one fused kernel where
 /// mc_morpho_pair_forward covers the case and two mc_morpho_forward calls otherwise; the backward pass is the two
-/// mc_morpho_backward calls the separate operators would make (winners recomputed: no index is kept), their input
-/// gradients added and the erosion's weight gradient flipped back (erosion works on the flipped structuring element,
-/// morphocore/functional/erosion.py:89).
+/// mc_morpho_backward calls the separate operators would make (winners recomputed: no index is kept), the second of which
+/// adds to the gradients of the first.
 class MorphoPairFunction : public torch::autograd::Function<MorphoPairFunction>
 {
 public:
@@ -291,7 +293,7 @@ public:
                                                 int64_t padding, double padding_value)
     {
         const MorphoPairCall call = run_morpho_pair_forward(input, weight, merge, padding, padding_value);
-        ctx->save_for_backward({call.input4d, call.weight4d, call.flipped});
+        ctx->save_for_backward({call.input4d, call.weight4d});
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["padding"] = padding;
         ctx->saved_data["padding_value"] = padding_value;
@@ -305,7 +307,6 @@ public:
         const auto saved = ctx->get_saved_variables();
         const torch::Tensor& input = saved[0];
         const torch::Tensor& weight = saved[1];
-        const torch::Tensor& flipped = saved[2];
         const int64_t merge = ctx->saved_data["merge"].toInt(), padding = ctx->saved_data["padding"].toInt();
         const double padding_value = ctx->saved_data["padding_value"].toDouble();
         const c10::cuda::CUDAGuard device_guard(input.device());
@@ -326,17 +327,19 @@ public:
             mc_desc d = make_desc(input, weight, op, merge);
             d.pad_kind = padding == PAD_REPLICATE ? MC_PAD_REPLICATE : MC_PAD_FILL;
             d.fill = fill_value(op, padding, padding_value, d.dtype == MC_F32);
-            const torch::Tensor& kernel_weight = op == MC_OP_DILATION ? weight : flipped;
-            torch::Tensor gx = torch::empty_like(input), gw = torch::empty_like(weight);
+            // Erosion works on the flipped structuring element; the second half adds to the gradients of the first.
+            d.flags = (op == MC_OP_EROSION ? MC_FLAG_FLIPPED_WEIGHT : 0) | (grad_input.defined() ? MC_FLAG_ACCUMULATE : 0);
+            if (!grad_input.defined())
+            {
+                grad_input = at::empty_like(input);
+                grad_weight = at::empty_like(weight);
+            }
             const size_t ws_bytes = mc_morpho_backward_workspace_bytes(&d, 0);
             torch::Tensor workspace;
             if (ws_bytes > 0) workspace = torch::empty({static_cast<int64_t>(ws_bytes)}, input.options().dtype(torch::kByte));
             const TraceRange trace("morphocore::morpho_backward");
-            check_status(mc_morpho_backward(&d, input.data_ptr(), kernel_weight.data_ptr(), nullptr, grad_output.data_ptr(), gx.data_ptr(), gw.data_ptr(),
-                                            workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, stream));
-            if (op == MC_OP_EROSION) gw = gw.flip({2, 3});
-            grad_input = grad_input.defined() ? grad_input + gx : gx;
-            grad_weight = grad_weight.defined() ? grad_weight + gw : gw;
+            check_status(mc_morpho_backward(&d, input.data_ptr(), weight.data_ptr(), nullptr, grad_output.data_ptr(), grad_input.data_ptr(),
+                                            grad_weight.data_ptr(), workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, stream));
         }
         if (grad_input.defined())
         {
@@ -360,10 +363,19 @@ torch::Tensor pair_alphas(const torch::Tensor& alpha, int64_t merge, int64_t out
 /// One forward smorph and what its backward pass needs.
 struct SmorphCall
 {
-    torch::Tensor input4d, weight4d, output;
+    torch::Tensor input4d, weight4d, alphas, output;
+    torch::Tensor raw_weight;   // the structuring element before the re-parametrisation, where the call includes it
 };
 
-SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, int64_t merge)
+/// w~ of the pairs (mc_smorph_reparametrise).
+torch::Tensor reparametrised(const mc_desc& d, const torch::Tensor& weight4d, const torch::Tensor& alphas, cudaStream_t stream)
+{
+    torch::Tensor out = at::empty_like(weight4d);
+    check_status(mc_smorph_reparametrise(&d, weight4d.data_ptr(), alphas.data_ptr(), out.data_ptr(), stream));
+    return out;
+}
+
+SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, int64_t merge, bool reparametrise)
 {
     SmorphCall call;
     call.input4d = input_to_4d(input);
@@ -388,25 +400,43 @@ SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& w
     const c10::cuda::CUDAGuard device_guard(input.device());
     call.input4d = call.input4d.contiguous();
     call.weight4d = call.weight4d.contiguous();
-    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
-    const torch::Tensor alphas = pair_alphas(alpha, merge, weight4d.size(0), input4d.size(1));
+    const torch::Tensor& input4d = call.input4d;
+    call.alphas = pair_alphas(alpha, merge, call.weight4d.size(0), input4d.size(1));
 
-    const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, merge);
-    call.output = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    const mc_desc d = make_desc(input4d, call.weight4d, MC_OP_DILATION, merge);
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const TraceRange trace("morphocore::smorph_forward");
-    check_status(mc_smorph_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), call.output.data_ptr(),
-                                   at::cuda::getCurrentCUDAStream().stream()));
+    if (reparametrise)
+    {
+        call.raw_weight = call.weight4d;
+        call.weight4d = reparametrised(d, call.raw_weight, call.alphas, stream);
+    }
+    call.output = at::empty({input4d.size(0), call.weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    check_status(mc_smorph_forward(&d, input4d.data_ptr(), call.weight4d.data_ptr(), call.alphas.data_ptr(), call.output.data_ptr(), stream));
     return call;
+}
+
+/// Gradient of the structuring element as the user holds it, from that of w~; adds to the alpha gradient what flows through
+/// w~. Returns `grad` itself where the call had no re-parametrisation.
+torch::Tensor through_reparametrisation(const mc_desc& d, const torch::Tensor& raw_weight, const torch::Tensor& alphas, const torch::Tensor& grad,
+                                        torch::Tensor& grad_alpha_pairs, cudaStream_t stream)
+{
+    if (!raw_weight.defined()) return grad;
+    torch::Tensor out = at::empty_like(grad);
+    check_status(mc_smorph_reparametrise_backward(&d, raw_weight.data_ptr(), alphas.data_ptr(), grad.data_ptr(), out.data_ptr(),
+                                                  grad_alpha_pairs.data_ptr(), stream));
+    return out;
 }
 
 class SmorphFunction : public torch::autograd::Function<SmorphFunction>
 {
 public:
-    static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, int64_t merge)
+    static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, int64_t merge,
+                                 bool reparametrise)
     {
-        const SmorphCall call = run_smorph_forward(input, weight, alpha, merge);
+        const SmorphCall call = run_smorph_forward(input, weight, alpha, merge, reparametrise);
         // The backward pass reads the 4-D output: the merge target of MAX and MIN.
-        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d});
+        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d, call.alphas, call.raw_weight});
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
@@ -420,6 +450,8 @@ public:
         const torch::Tensor& alpha = saved[1];
         const torch::Tensor& input = saved[2];
         const torch::Tensor& weight = saved[3];
+        const torch::Tensor& alphas = saved[4];
+        const torch::Tensor& raw_weight = saved[5];
         const int64_t merge = ctx->saved_data["merge"].toInt();
         torch::Tensor grad_output = input_to_4d(grad_outputs[0]).contiguous();
         TORCH_CHECK(grad_output.sizes() == output.sizes(), "grad_output shape mismatch: expected [", output.sizes(), "] but got [",
@@ -429,7 +461,6 @@ public:
 
         const c10::cuda::CUDAGuard device_guard(input.device());
         const mc_desc d = make_desc(input, weight, MC_OP_DILATION, merge);
-        const torch::Tensor alphas = pair_alphas(alpha, merge, weight.size(0), input.size(1));
         torch::Tensor grad_input = torch::empty_like(input);
         torch::Tensor grad_weight = torch::empty_like(weight);
         torch::Tensor grad_alpha_pairs = torch::empty_like(alphas);
@@ -438,26 +469,30 @@ public:
         if (ws_bytes > 0) workspace = torch::empty({static_cast<int64_t>(ws_bytes)}, input.options().dtype(torch::kByte));
 
         const TraceRange trace("morphocore::smorph_backward");
+        const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
         check_status(mc_smorph_backward(&d, input.data_ptr(), weight.data_ptr(), alphas.data_ptr(), output.data_ptr(), grad_output.data_ptr(),
                                         grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
-                                        workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, at::cuda::getCurrentCUDAStream().stream()));
+                                        workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, stream));
+        grad_weight = through_reparametrisation(d, raw_weight, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph.cpp:96-98).
         torch::Tensor grad_alpha =
             alpha.numel() == grad_alpha_pairs.numel() ? grad_alpha_pairs.view_as(alpha) : grad_alpha_pairs.sum().view_as(alpha);
         grad_input = output_to_original(grad_input, ctx->saved_data["input_dims"].toInt());
         if (ctx->saved_data["weight_dims"].toInt() == 2) grad_weight = grad_weight.squeeze(0).squeeze(0);
-        return {grad_input, grad_weight, grad_alpha, torch::Tensor()};
+        return {grad_input, grad_weight, grad_alpha, torch::Tensor(), torch::Tensor()};
     }
 };
 
 /// One forward smorph with the smooth channel merge and what its backward pass needs.
 struct SmorphScmCall
 {
-    torch::Tensor input4d, weight4d, betas, output;
+    torch::Tensor input4d, weight4d, alphas, betas, output;
+    torch::Tensor raw_weight;   // as in SmorphCall
 };
 
-SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, const torch::Tensor& beta)
+SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, const torch::Tensor& beta,
+                                     bool reparametrise)
 {
     SmorphScmCall call;
     call.input4d = input_to_4d(input);
@@ -477,14 +512,20 @@ SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Te
     call.input4d = call.input4d.contiguous();
     call.weight4d = call.weight4d.contiguous();
     call.betas = beta.contiguous();
-    const torch::Tensor &input4d = call.input4d, &weight4d = call.weight4d;
-    const torch::Tensor alphas = pair_alphas(alpha, MC_MERGE_SMOOTH, weight4d.size(0), input4d.size(1));
+    const torch::Tensor& input4d = call.input4d;
+    call.alphas = pair_alphas(alpha, MC_MERGE_SMOOTH, call.weight4d.size(0), input4d.size(1));
 
-    const mc_desc d = make_desc(input4d, weight4d, MC_OP_DILATION, MC_MERGE_SMOOTH);
-    call.output = at::empty({input4d.size(0), weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    const mc_desc d = make_desc(input4d, call.weight4d, MC_OP_DILATION, MC_MERGE_SMOOTH);
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const TraceRange trace("morphocore::smorph_scm_forward");
-    check_status(mc_smorph_scm_forward(&d, input4d.data_ptr(), weight4d.data_ptr(), alphas.data_ptr(), call.betas.data_ptr(), call.output.data_ptr(),
-                                       at::cuda::getCurrentCUDAStream().stream()));
+    if (reparametrise)
+    {
+        call.raw_weight = call.weight4d;
+        call.weight4d = reparametrised(d, call.raw_weight, call.alphas, stream);
+    }
+    call.output = at::empty({input4d.size(0), call.weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
+    check_status(mc_smorph_scm_forward(&d, input4d.data_ptr(), call.weight4d.data_ptr(), call.alphas.data_ptr(), call.betas.data_ptr(),
+                                       call.output.data_ptr(), stream));
     return call;
 }
 
@@ -494,11 +535,11 @@ class SmorphScmFunction : public torch::autograd::Function<SmorphScmFunction>
 {
 public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, torch::Tensor alpha,
-                                 torch::Tensor beta)
+                                 torch::Tensor beta, bool reparametrise)
     {
-        const SmorphScmCall call = run_smorph_scm_forward(input, weight, alpha, beta);
+        const SmorphScmCall call = run_smorph_scm_forward(input, weight, alpha, beta, reparametrise);
         // The backward pass reads the 4-D output: the final value of the soft merge.
-        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d});
+        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d, call.alphas, call.raw_weight});
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
         return output_to_original(call.output, input.dim());
@@ -512,6 +553,8 @@ public:
         const torch::Tensor& beta = saved[2];
         const torch::Tensor& input = saved[3];
         const torch::Tensor& weight = saved[4];
+        const torch::Tensor& alphas = saved[5];
+        const torch::Tensor& raw_weight = saved[6];
         torch::Tensor grad_output = input_to_4d(grad_outputs[0]).contiguous();
         TORCH_CHECK(grad_output.sizes() == output.sizes(), "grad_output shape mismatch: expected [", output.sizes(), "] but got [",
                     grad_output.sizes(), "]");
@@ -520,7 +563,6 @@ public:
 
         const c10::cuda::CUDAGuard device_guard(input.device());
         const mc_desc d = make_desc(input, weight, MC_OP_DILATION, MC_MERGE_SMOOTH);
-        const torch::Tensor alphas = pair_alphas(alpha, MC_MERGE_SMOOTH, weight.size(0), input.size(1));
         torch::Tensor grad_input = torch::empty_like(input);
         torch::Tensor grad_weight = torch::empty_like(weight);
         torch::Tensor grad_alpha_pairs = torch::empty_like(alphas);
@@ -528,16 +570,18 @@ public:
         const size_t ws_bytes = mc_smorph_scm_backward_workspace_bytes(&d);
         torch::Tensor workspace = torch::empty({static_cast<int64_t>(ws_bytes)}, input.options().dtype(torch::kByte));
         const TraceRange trace("morphocore::smorph_scm_backward");
+        const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
         check_status(mc_smorph_scm_backward(&d, input.data_ptr(), weight.data_ptr(), alphas.data_ptr(), beta.data_ptr(), output.data_ptr(),
                                             grad_output.data_ptr(), grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
-                                            grad_beta.data_ptr(), workspace.data_ptr(), ws_bytes, at::cuda::getCurrentCUDAStream().stream()));
+                                            grad_beta.data_ptr(), workspace.data_ptr(), ws_bytes, stream));
+        grad_weight = through_reparametrisation(d, raw_weight, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph_scm.cpp:81-83).
         torch::Tensor grad_alpha =
             alpha.numel() == grad_alpha_pairs.numel() ? grad_alpha_pairs.view_as(alpha) : grad_alpha_pairs.sum().view_as(alpha);
         grad_input = output_to_original(grad_input, ctx->saved_data["input_dims"].toInt());
         if (ctx->saved_data["weight_dims"].toInt() == 2) grad_weight = grad_weight.squeeze(0).squeeze(0);
-        return {grad_input, grad_weight, grad_alpha, grad_beta};
+        return {grad_input, grad_weight, grad_alpha, grad_beta, torch::Tensor()};
     }
 };
 
@@ -567,11 +611,11 @@ torch::Tensor widen(const torch::Tensor& t, const torch::Tensor& like, const cha
 }
 
 torch::Tensor morpho_call(const torch::Tensor& input, const torch::Tensor& weight, int64_t op, int64_t merge, int64_t padding, double padding_value,
-                          bool save_indices, double noise_scale)
+                          bool save_indices, double noise_scale, int64_t flags = 0)
 {
-    if (differentiated({&input, &weight})) return MorphoFunction::apply(input, weight, op, merge, padding, padding_value, save_indices, noise_scale);
+    if (differentiated({&input, &weight})) return MorphoFunction::apply(input, weight, op, merge, padding, padding_value, save_indices, noise_scale, flags);
     const at::AutoDispatchBelowADInplaceOrView guard;
-    return output_to_original(run_morpho_forward(input, weight, op, merge, padding, padding_value, false, noise_scale).output, input.dim());
+    return output_to_original(run_morpho_forward(input, weight, op, merge, padding, padding_value, false, noise_scale, flags).output, input.dim());
 }
 
 torch::Tensor dilation(torch::Tensor input, torch::Tensor weight, int64_t merge, int64_t padding, double padding_value, bool save_indices,
@@ -592,6 +636,16 @@ torch::Tensor erosion(torch::Tensor input, torch::Tensor weight, int64_t merge, 
     return morpho_call(input, weight, MC_OP_EROSION, checked_merge(merge), checked_padding(padding), padding_value, save_indices, noise_scale);
 }
 
+/// Extension (not an operator of the reference): erosion with the structuring element as the user holds it. The kernels read
+/// it, and write its gradient, with both axes reversed, instead of working on a flipped copy (two launches and an autograd
+/// node less).
+torch::Tensor erosion_layer(torch::Tensor input, torch::Tensor weight, int64_t merge, int64_t padding, double padding_value, bool save_indices)
+{
+    if (is_reduced(input))
+        return erosion_layer(input.to(torch::kFloat), widen(weight, input, "weight"), merge, padding, padding_value, save_indices).to(input.scalar_type());
+    return morpho_call(input, weight, MC_OP_EROSION, checked_merge(merge), checked_padding(padding), padding_value, save_indices, 0.0, MC_FLAG_FLIPPED_WEIGHT);
+}
+
 /// Extension (not an operator of the reference): both halves of sigma_layer at once. MAX / MIN merges that keep their
 /// winner indices for the backward pass run the two separate operators, which is what saves them.
 std::tuple<torch::Tensor, torch::Tensor> dilation_erosion(torch::Tensor input, torch::Tensor weight, int64_t merge, int64_t padding, double padding_value,
@@ -606,7 +660,7 @@ std::tuple<torch::Tensor, torch::Tensor> dilation_erosion(torch::Tensor input, t
     padding = checked_padding(padding);
     if (save_indices && (merge == MC_MERGE_MAX || merge == MC_MERGE_MIN) && differentiated({&input, &weight}))
         return {dilation(input, weight, merge, padding, padding_value, true, 0.0),
-                erosion(input, weight.flip({-2, -1}), merge, padding, padding_value, true, 0.0)};
+                erosion_layer(input, weight, merge, padding, padding_value, true)};
     if (!differentiated({&input, &weight}))
     {
         const at::AutoDispatchBelowADInplaceOrView guard;
@@ -617,14 +671,33 @@ std::tuple<torch::Tensor, torch::Tensor> dilation_erosion(torch::Tensor input, t
     return {out[0], out[1]};
 }
 
-torch::Tensor smorph(torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, int64_t merge)
+torch::Tensor smorph_call(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, int64_t merge, bool reparametrise)
+{
+    if (differentiated({&input, &weight, &alpha})) return SmorphFunction::apply(input, weight, alpha, merge, reparametrise);
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return output_to_original(run_smorph_forward(input, weight, alpha, merge, reparametrise).output, input.dim());
+}
+
+torch::Tensor smorph_scm_call(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, const torch::Tensor& beta,
+                              bool reparametrise)
+{
+    if (differentiated({&input, &weight, &alpha, &beta})) return SmorphScmFunction::apply(input, weight, alpha, beta, reparametrise);
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return output_to_original(run_smorph_scm_forward(input, weight, alpha, beta, reparametrise).output, input.dim());
+}
+
+int64_t checked_smorph_merge(int64_t merge)
 {
     TORCH_CHECK(merge >= 0 && merge <= MC_MERGE_IDENTITY && merge != MC_MERGE_SMOOTH, "Unsupported merge operation for smorph");
+    return merge;
+}
+
+torch::Tensor smorph(torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, int64_t merge)
+{
+    checked_smorph_merge(merge);
     if (is_reduced(input))
         return smorph(input.to(torch::kFloat), widen(weight, input, "weight"), widen(alpha, input, "alpha"), merge).to(input.scalar_type());
-    if (differentiated({&input, &weight, &alpha})) return SmorphFunction::apply(input, weight, alpha, merge);
-    const at::AutoDispatchBelowADInplaceOrView guard;
-    return output_to_original(run_smorph_forward(input, weight, alpha, merge).output, input.dim());
+    return smorph_call(input, weight, alpha, merge, false);
 }
 
 torch::Tensor smorph_scm(torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, torch::Tensor beta)
@@ -632,9 +705,44 @@ torch::Tensor smorph_scm(torch::Tensor input, torch::Tensor weight, torch::Tenso
     if (is_reduced(input))
         return smorph_scm(input.to(torch::kFloat), widen(weight, input, "weight"), widen(alpha, input, "alpha"), widen(beta, input, "beta"))
             .to(input.scalar_type());
-    if (differentiated({&input, &weight, &alpha, &beta})) return SmorphScmFunction::apply(input, weight, alpha, beta);
-    const at::AutoDispatchBelowADInplaceOrView guard;
-    return output_to_original(run_smorph_scm_forward(input, weight, alpha, beta).output, input.dim());
+    return smorph_scm_call(input, weight, alpha, beta, false);
+}
+
+/// Whether the re-parametrisation kernel covers these arguments: one alpha per pair in its natural shape, or a single one.
+/// Everything else (also what the operators reject with a message of their own) takes the chain of tensor operations.
+bool kernel_reparametrises(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, bool identity, bool smooth)
+{
+    if (weight.dim() != 4 || alpha.dim() > 2 || !weight.is_cuda() || weight.device() != alpha.device() || weight.device() != input.device()) return false;
+    if (weight.scalar_type() != alpha.scalar_type() || weight.scalar_type() != input.scalar_type() || weight.numel() == 0) return false;
+    if (weight.scalar_type() != torch::kFloat && weight.scalar_type() != torch::kDouble) return false;
+    if (alpha.numel() == 1) return true;
+    const int64_t out = weight.size(0), in = weight.size(1);
+    if (identity) return !smooth && in == 1 && alpha.numel() == out;
+    return alpha.dim() == 2 ? alpha.size(0) == out && alpha.size(1) == in : in == 1 && alpha.numel() == out;
+}
+
+/// Extension (not an operator of the reference): functional.smorph as a whole, the re-parametrisation of the structuring
+/// element (morphocore/functional/smorph.py:60-68) included. As a chain of tensor operations that is ten launches forward
+/// and eighteen backward, 80 and 150 us of host time around kernels that take 20 us on small feature maps; here it is one
+/// launch each way. `beta` selects the smooth channel merge; `merge` IDENTITY then only says how alpha is shaped.
+torch::Tensor smorph_layer(torch::Tensor input, torch::Tensor weight, torch::Tensor alpha, const std::optional<torch::Tensor>& beta, int64_t merge)
+{
+    const bool smooth = beta.has_value() && beta->defined();
+    checked_smorph_merge(merge);
+    if (is_reduced(input))
+    {
+        std::optional<torch::Tensor> wide_beta;
+        if (smooth) wide_beta = widen(*beta, input, "beta");
+        return smorph_layer(input.to(torch::kFloat), widen(weight, input, "weight"), widen(alpha, input, "alpha"), wide_beta, merge)
+            .to(input.scalar_type());
+    }
+    const bool identity = merge == MC_MERGE_IDENTITY;
+    if (kernel_reparametrises(input, weight, alpha, identity, smooth))
+        return smooth ? smorph_scm_call(input, weight, alpha, *beta, true) : smorph_call(input, weight, alpha, merge, true);
+    torch::Tensor t = torch::tanh(alpha);
+    t = identity || alpha.dim() == 1 ? t.view({-1, 1, 1, 1}) : t.unsqueeze(-1).unsqueeze(-1);
+    const torch::Tensor tilde = t * ((1 - t) / 2 * weight.flip({-2, -1}) + (1 + t) / 2 * weight);
+    return smooth ? smorph_scm(input, tilde, alpha, *beta) : smorph(input, tilde, alpha, merge);
 }
 
 }  // namespace
@@ -648,6 +756,8 @@ TORCH_LIBRARY(morphocore, m)
     m.def("smorph(Tensor input, Tensor weight, Tensor alpha, int merge) -> Tensor");
     m.def("smorph_scm(Tensor input, Tensor weight, Tensor alpha, Tensor beta) -> Tensor");
     m.def("dilation_erosion(Tensor input, Tensor weight, int merge, int padding, float padding_value=0., bool save_indices=True) -> (Tensor, Tensor)");
+    m.def("smorph_layer(Tensor input, Tensor weight, Tensor alpha, Tensor? beta, int merge) -> Tensor");
+    m.def("erosion_layer(Tensor input, Tensor weight, int merge, int padding, float padding_value=0., bool save_indices=True) -> Tensor");
 }
 
 TORCH_LIBRARY_IMPL(morphocore, CompositeImplicitAutograd, m)
@@ -657,4 +767,6 @@ TORCH_LIBRARY_IMPL(morphocore, CompositeImplicitAutograd, m)
     m.impl("smorph", &smorph);
     m.impl("smorph_scm", &smorph_scm);
     m.impl("dilation_erosion", &dilation_erosion);
+    m.impl("smorph_layer", &smorph_layer);
+    m.impl("erosion_layer", &erosion_layer);
 }

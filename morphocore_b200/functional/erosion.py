@@ -15,12 +15,14 @@ def erosion(x: torch.Tensor, w: torch.Tensor, channel_merge_mode: str = 'sum',
     wf = w flipped along both kernel axes.
 
     Same signature and semantics as the reference `morphocore.functional.erosion`
-    (morphocore/functional/erosion.py:5-91): the operator receives the flipped structuring element and
-    autograd un-flips its gradient. 'geodesic' padding reads +inf. Dropped weights are -inf, so that
+    (morphocore/functional/erosion.py:5-91): the kernels read the structuring element, and write
+    its gradient, with both axes reversed. 'geodesic' padding reads +inf. Dropped weights are -inf, so that
     x - (-inf) = +inf never wins the minimum. See `dilation` for the arguments.
     """
     if training and weight_dropout > 0.0:
         w = drop_weights(w, weight_dropout)
+    if not training or noise_scale == 0.0:
+        return ops.erosion_layer(x, w, str_to_merge(channel_merge_mode), str_to_padding(padding_mode), padding_value, save_indices)
+    # The per-sample noise is drawn for the flipped structuring element.
     return ops.erosion(x, w.flip((-2, -1)), str_to_merge(channel_merge_mode),
-                       str_to_padding(padding_mode), padding_value, save_indices,
-                       noise_scale if training else 0.0)
+                       str_to_padding(padding_mode), padding_value, save_indices, noise_scale)

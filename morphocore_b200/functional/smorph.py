@@ -1,7 +1,7 @@
 import torch
 
 from ._ops import ops
-from .merge_enum import str_to_merge
+from .merge_enum import MorphoMerge, str_to_merge
 
 
 def smorph(x: torch.Tensor, w: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor = None,
@@ -10,7 +10,7 @@ def smorph(x: torch.Tensor, w: torch.Tensor, alpha: torch.Tensor, beta: torch.Te
     erosion as alpha -> -inf, on the GPU.
 
     Same signature and semantics as the reference `morphocore.functional.smorph`
-    (morphocore/functional/smorph.py:6-75). The structuring element is first re-parametrised in PyTorch,
+    (morphocore/functional/smorph.py:6-75). The structuring element is first re-parametrised, by a small kernel of its own,
 
         w~(alpha) = tanh(alpha) * ( (1 - tanh alpha)/2 * flip(w) + (1 + tanh alpha)/2 * w ),
 
@@ -24,15 +24,9 @@ def smorph(x: torch.Tensor, w: torch.Tensor, alpha: torch.Tensor, beta: torch.Te
         i, out = sum_i softmax_i(beta c_i) c_i (reference: morphocore/functional/csrc/cpp/smorph_scm.cpp:13-56).
     channel_merge_mode : 'sum', 'max', 'min', 'mean' or 'identity'.
     """
-    if channel_merge_mode == 'identity' or alpha.dim() == 1:
-        tanh_alpha = torch.tanh(alpha).view(-1, 1, 1, 1)
-    else:
-        tanh_alpha = torch.tanh(alpha).unsqueeze(-1).unsqueeze(-1)
-
-    term1 = (1 + tanh_alpha) / 2
-    term2 = (1 - tanh_alpha) / 2
-    w_tilde_alpha = tanh_alpha * (term2 * w.flip(dims=(-2, -1)) + term1 * w)
-
     if beta is not None:
-        return ops.smorph_scm(x, w_tilde_alpha, alpha, beta)
-    return ops.smorph(x, w_tilde_alpha, alpha, str_to_merge(channel_merge_mode))
+        # The channel merge is the smooth one: of the mode, only 'identity' matters, for the shape of alpha.
+        merge = MorphoMerge.IDENTITY if channel_merge_mode == 'identity' else MorphoMerge.ADD
+    else:
+        merge = str_to_merge(channel_merge_mode)
+    return ops.smorph_layer(x, w, alpha, beta, merge)

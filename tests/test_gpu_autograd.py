@@ -347,3 +347,55 @@ def test_compositions(F):
     layer = Mnn.SigmaLayer(3, 4, 3).cuda()
     layer(x).sum().backward()
     assert layer.alpha.grad is not None and layer.weight.grad is not None
+
+
+@pytest.mark.parametrize("merge", ["sum", "max", "identity"])
+@pytest.mark.parametrize("k", [(3, 3), (5, 5), (7, 7), (4, 3), (11, 11)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_erosion_reads_the_structuring_element_reversed(F, merge, k, dtype):
+    """functional.erosion hands the kernels the structuring element as the user holds it; the operator on a flipped copy is the
+    definition. Outputs are the same bits; gradients are sums of the same terms in another order: n terms of one size round to
+    n eps at the most, and the largest sum here (a weight gradient over 2 x 40 x 70 pixels) stays under 1e-4 of its largest
+    entry in float."""
+    torch.manual_seed(3)
+    x = torch.rand(2, 9, 40, 70, dtype=dtype, device="cuda")
+    w = 0.1 * torch.randn(9 if merge == "identity" else 5, 1 if merge == "identity" else 9, *k, dtype=dtype, device="cuda")
+    gy = torch.randn(2, w.shape[0], 40, 70, dtype=dtype, device="cuda")
+    got = [t.clone().requires_grad_(True) for t in (x, w)]
+    want = [t.clone().requires_grad_(True) for t in (x, w)]
+    y = F.erosion(*got, merge, "zero")
+    z = torch.ops.morphocore.erosion(want[0], want[1].flip((-2, -1)), {"max": 0, "sum": 2, "identity": 5}[merge], 0, 0.0, True, 0.0)
+    assert torch.equal(y, z)
+    y.backward(gy)
+    z.backward(gy)
+    for a, b in zip(got, want):
+        assert (a.grad - b.grad).abs().max() <= (1e-4 if dtype == torch.float32 else 1e-12) * b.grad.abs().max()
+
+
+@pytest.mark.parametrize("shape", ["pairs", "single", "identity", "identity_1d", "smooth"])
+@pytest.mark.parametrize("k", [(1, 1), (3, 3), (7, 5), (11, 11)])
+def test_smorph_reparametrisation_kernel(F, shape, k):
+    """functional.smorph re-parametrises the structuring element in a kernel of its own; in double, values and gradients against
+    the chain of tensor operations (the definition, morphocore/functional/smorph.py:60-68). Same operations, sums of k terms."""
+    torch.manual_seed(4)
+    c, identity = 4, shape.startswith("identity")
+    leaf = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda").requires_grad_(True)   # noqa: E731
+    x, w = leaf(2, c, 13, 18), leaf(c if identity else 3, 1 if identity else c, *k)
+    a = leaf(1) if shape == "single" else leaf(c) if shape == "identity_1d" else leaf(c, 1) if identity else leaf(3, c)
+    beta = leaf(3) if shape == "smooth" else None
+    gy = torch.randn(2, w.shape[0], 13, 18, dtype=torch.float64, device="cuda")
+    leaves = [t for t in (x, w, a, beta) if t is not None]
+    merge = "identity" if identity else "sum"
+    y = F.smorph(x, w, a, beta, merge)
+    got = torch.autograd.grad(y, leaves, gy)
+    t = torch.tanh(a)
+    t = t.view(-1, 1, 1, 1) if identity or a.dim() == 1 else t[..., None, None]
+    tilde = t * ((1 - t) / 2 * w.flip((-2, -1)) + (1 + t) / 2 * w)
+    ops = torch.ops.morphocore
+    z = ops.smorph(x, tilde, a, 5 if identity else 2) if beta is None else ops.smorph_scm(x, tilde, a, beta)
+    want = torch.autograd.grad(z, leaves, gy)
+    assert torch.allclose(y, z, rtol=1e-12, atol=1e-12)
+    for p, q in zip(got, want):
+        assert p.shape == q.shape and (p - q).abs().max() <= 1e-11 * q.abs().max().clamp_min(1.0)
+    with torch.no_grad():
+        assert torch.equal(F.smorph(x, w, a, beta, merge), y)
