@@ -217,6 +217,77 @@ __device__ __forceinline__ void stage_window_async(T* __restrict__ dst, const T*
     }
 }
 
+/// Window rows / columns that the live warps of a tile can read (thread_patch: a warp whose 32 x 8 block lies outside the
+/// image does no arithmetic).
+__device__ __forceinline__ int live_window_rows(const Geometry& g, int tile_h0)
+{
+    return g.win_rows - 8 * (TILE_H / 8 - (min(g.H - tile_h0, TILE_H) + 7) / 8);
+}
+__device__ __forceinline__ int live_window_cols(const Geometry& g, int tile_w0)
+{
+    return g.win_stride - 32 * (TILE_W / 32 - (min(g.W - tile_w0, TILE_W) + 31) / 32);
+}
+
+/// The windows of `channels` consecutive planes of one tile, border resolved, by asynchronous copies of single elements: for
+/// tensors whose rows TMA cannot address (a row pitch that is no multiple of 16 bytes: any odd width). A thread's columns and
+/// their clamping are the same for every row and channel and are computed once. STRIDE is the row stride, 0 for the one in
+/// `g`. The caller waits (cp_async_wait_all) and synchronises the CTA before the windows are read.
+template <int STRIDE, typename T>
+__device__ __forceinline__ void stage_windows_async(T* __restrict__ dst, const T* __restrict__ planes, int channels, const Geometry& g, int tile_h0,
+                                                    int tile_w0, T outside)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row0 = tile_h0 - g.halo_top(), col0 = tile_w0 - g.halo_left();
+    const int rows = live_window_rows(g, tile_h0), cols = live_window_cols(g, tile_w0);
+    const int64_t plane = g.plane();
+    auto copy_row = [&](T* out, const T* src, bool row_in, int c, int column, bool column_in) {
+        if (c < cols)
+        {
+            if (row_in && column_in) cp_async_element(out + c, src + column);
+            else out[c] = outside;
+        }
+    };
+    if constexpr (STRIDE > 0)
+    {
+        constexpr int M = (STRIDE + 31) / 32;
+        int column[M];
+        bool column_in[M];
+#pragma unroll
+        for (int m = 0; m < M; m++)
+        {
+            const int ix = col0 + lane + 32 * m;
+            column[m] = min(max(ix, 0), g.W - 1);
+            column_in[m] = g.replicate || (ix >= 0 && ix < g.W);
+        }
+        for (int r = warp; r < rows; r += THREADS / 32)
+        {
+            const int iy = row0 + r;
+            const bool row_in = g.replicate || (iy >= 0 && iy < g.H);
+            const T* src = planes + static_cast<int64_t>(min(max(iy, 0), g.H - 1)) * g.W;
+            T* out = dst + r * STRIDE;
+            for (int c = 0; c < channels; c++, src += plane, out += g.win_rows * STRIDE)
+#pragma unroll
+                for (int m = 0; m < M; m++) copy_row(out, src, row_in, lane + 32 * m, column[m], column_in[m]);
+        }
+    }
+    else
+    {
+        for (int r = warp; r < rows; r += THREADS / 32)
+        {
+            const int iy = row0 + r;
+            const bool row_in = g.replicate || (iy >= 0 && iy < g.H);
+            const T* src = planes + static_cast<int64_t>(min(max(iy, 0), g.H - 1)) * g.W;
+            T* out = dst + r * g.win_stride;
+            for (int c = 0; c < channels; c++, src += plane, out += g.window_elems())
+                for (int m = lane; m < cols; m += 32)
+                {
+                    const int ix = col0 + m;
+                    copy_row(out, src, row_in, m, min(max(ix, 0), g.W - 1), g.replicate || (ix >= 0 && ix < g.W));
+                }
+        }
+    }
+}
+
 /// Stage the window of one plane for the smorph kernels, whose taps outside the image are excluded. Both
 /// windows hold x inside the image; outside, `low` (read by pairs with alpha >= 0, u = x + w) holds -big and
 /// `high` (read by pairs with alpha < 0, u = -x - w) holds +big, so that u = -big there: a value that never
@@ -279,6 +350,14 @@ template <bool IS_MIN> __device__ __forceinline__ float ext3(float a, float b, f
     if (IS_MIN) asm("min.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(b), "f"(c));
     else asm("max.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(b), "f"(c));
     return a;
+}
+/// ext3 of a value that stays live (a constant): the result has a register of its own.
+template <bool IS_MIN> __device__ __forceinline__ float ext3_of(float a, float b, float c)
+{
+    float r;
+    if (IS_MIN) asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    else asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 template <bool IS_MIN> __device__ __forceinline__ double ext3(double a, double b, double c) { return ext2<IS_MIN>(ext2<IS_MIN>(a, b), c); }
 

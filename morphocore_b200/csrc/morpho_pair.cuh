@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_pair_forward_kernel(const P
             if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
             return;  // every thread of the CTA waits on the same barrier and gives up together
         }
-        if (fix_border) fix_window_border(sx, xb + static_cast<int64_t>(first_channel + c0) * plane, plane, cc, g, tile_h0, tile_w0, a.fill);
+        if (fix_border) fix_window_border(sx, cc, g, tile_h0, tile_w0, a.fill);
         __syncthreads();
 
         for (int c = 0; c < cc && warp_live; c++)

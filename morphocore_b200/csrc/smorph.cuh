@@ -999,9 +999,9 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
             if (border)
             {
                 const T* src = xb + static_cast<int64_t>(first_channel + c0) * plane;
-                fix_window_border(stage, src, plane, min(cc, a.chunk), g, tile_h0, tile_w0, fill0);
-                if (mixed) fix_window_border(stage + slot_elems, src, plane, cc, g, tile_h0, tile_w0, Limits<T>::big());
-                else if (cc > a.chunk) fix_window_border(stage + slot_elems, src + a.chunk * plane, plane, cc - a.chunk, g, tile_h0, tile_w0, fill0);
+                fix_window_border(stage, min(cc, a.chunk), g, tile_h0, tile_w0, fill0);
+                if (mixed) fix_window_border(stage + slot_elems, cc, g, tile_h0, tile_w0, Limits<T>::big());
+                else if (cc > a.chunk) fix_window_border(stage + slot_elems, cc - a.chunk, g, tile_h0, tile_w0, fill0);
             }
         }
         __syncthreads();

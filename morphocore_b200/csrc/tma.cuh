@@ -108,50 +108,42 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
                  : "memory");
 }
 
-/// After a TMA copy of a window (zero filled outside the image): overwrite the out-of-image elements of
-/// `channels` staged windows with the border rule. Only CTAs whose window leaves the image call this.
-/// Only the part of the window that a live warp can read is visited (see thread_patch: the warps of a
-/// partial tile whose 32 x 8 block lies outside the image do no arithmetic), which for the half-empty last
-/// tile column of a 224-wide image is 4 columns instead of 36.
+/// After a TMA copy of windows (zero filled outside the image): overwrite the out-of-image elements of `channels` staged
+/// windows with the border rule. Only CTAs whose window leaves the image call this, and only the part that a live warp can
+/// read is visited. The edge pixels of the REPLICATE rule are read from the window itself, which holds every pixel that the
+/// clamp can name (the clamped pixel of an out-of-image element lies at the near edge of the image, beside elements that
+/// live warps read): no global load stands between the copy and the arithmetic. Image elements are only read, the others
+/// only written, so no barrier is needed inside.
 template <typename T>
-__device__ __forceinline__ void fix_window_border(T* __restrict__ win, const T* __restrict__ planes, int64_t plane_stride, int channels,
-                                                  const Geometry& g, int tile_h0, int tile_w0, T outside)
+__device__ __forceinline__ void fix_window_border(T* __restrict__ win, int channels, const Geometry& g, int tile_h0, int tile_w0, T outside)
 {
     const int row0 = tile_h0 - g.halo_top(), col0 = tile_w0 - g.halo_left();
-    const int live_cols = g.win_stride - 32 * (TILE_W / 32 - (min(g.W - tile_w0, TILE_W) + 31) / 32);
-    const int live_rows = g.win_rows - 8 * (TILE_H / 8 - (min(g.H - tile_h0, TILE_H) + 7) / 8);
-    // Window rows [r_lo, r_hi) are image rows; of those, columns [0, n_left) and [first_right, live_cols) lie outside.
-    const int r_lo = min(max(-row0, 0), live_rows), r_hi = min(max(g.H - row0, 0), live_rows);
-    const int n_left = min(max(-col0, 0), live_cols);
-    const int first_right = min(max(g.W - col0, 0), live_cols);
-    const int n_side = n_left + live_cols - first_right;
-    const int welems = g.window_elems();
-    auto put = [&](int c, int wr, int col) {
-        T v = outside;
-        if (g.replicate)
-            v = __ldg(planes + c * plane_stride + static_cast<int64_t>(min(max(row0 + wr, 0), g.H - 1)) * g.W + min(max(col0 + col, 0), g.W - 1));
-        win[c * welems + wr * g.win_stride + col] = v;
-    };
+    const int rows = live_window_rows(g, tile_h0), cols = live_window_cols(g, tile_w0);
+    // Image part of the window: rows [r_lo, r_hi), columns [c_lo, c_hi); never empty (the tile has a pixel).
+    const int r_lo = max(-row0, 0), r_hi = min(g.H - row0, rows), c_lo = max(-col0, 0), c_hi = min(g.W - col0, cols);
+    const int stride = g.win_stride, welems = g.window_elems();
+    const int n_side = c_lo + cols - c_hi;
     if (n_side > 0)
     {
-        const int per_channel = (r_hi - r_lo) * n_side;
-        for (int e = threadIdx.x; e < channels * per_channel; e += THREADS)
-        {
-            const int c = e / per_channel, rest = e - c * per_channel;
-            const int r = rest / n_side, i = rest - r * n_side;
-            put(c, r_lo + r, i < n_left ? i : first_right + i - n_left);
-        }
+        // Eight lanes take a row of the image part: left and right columns.
+        for (int c = 0; c < channels; c++)
+            for (int r = r_lo + (threadIdx.x >> 3); r < r_hi; r += THREADS / 8)
+            {
+                T* row = win + c * welems + r * stride;
+                for (int i = threadIdx.x & 7; i < n_side; i += 8)
+                {
+                    const int col = i < c_lo ? i : c_hi + i - c_lo;
+                    row[col] = g.replicate ? row[i < c_lo ? c_lo : c_hi - 1] : outside;
+                }
+            }
     }
-    const int n_out = r_lo + live_rows - r_hi;   // rows above and below the image
-    if (n_out > 0)
+    const int n_out = r_lo + rows - r_hi;   // rows above and below the image: one per warp
+    for (int e = threadIdx.x >> 5; e < channels * n_out; e += THREADS / 32)
     {
-        const int per_channel = n_out * live_cols;
-        for (int e = threadIdx.x; e < channels * per_channel; e += THREADS)
-        {
-            const int c = e / per_channel, rest = e - c * per_channel;
-            const int r = rest / live_cols, col = rest - r * live_cols;
-            put(c, r < r_lo ? r : r_hi + r - r_lo, col);
-        }
+        const int c = e / n_out, i = e - c * n_out;
+        const T* edge = win + c * welems + (i < r_lo ? r_lo : r_hi - 1) * stride;
+        T* row = win + c * welems + (i < r_lo ? i : r_hi + i - r_lo) * stride;
+        for (int col = threadIdx.x & 31; col < cols; col += 32) row[col] = g.replicate ? edge[min(max(col, c_lo), c_hi - 1)] : outside;
     }
 }
 
