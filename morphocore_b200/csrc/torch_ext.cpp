@@ -5,6 +5,7 @@
 // lifted to 4-D, the same checks raise the same messages, the wrapper owns every allocation and the
 // kernels only write into caller buffers. There is no CPU path: CPU tensors are rejected.
 #include <nvtx3/nvToolsExt.h>
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/all.h>
@@ -100,15 +101,17 @@ double fill_value(int64_t op, int64_t padding, double padding_value, bool single
     return op == MC_OP_DILATION ? -std::numeric_limits<double>::infinity() : std::numeric_limits<double>::infinity();
 }
 
-/// Whether a call with these inputs will be differentiated. Calls that will not be (inference, or inputs that need no
-/// gradient) skip the autograd function, which saves about 2 us of host time, and the winner index of MAX / MIN merges,
+/// Whether a call with these inputs goes through the autograd function. Calls that will not be differentiated (inference, or
+/// inputs that need no gradient) skip it, which saves about 2 us of host time, and the winner index of MAX / MIN merges,
 /// whose only reader is the backward pass: on (8, 3, 128, 128) -> 16 channels the search for it took four fifths of the
-/// call (57 us with it).
+/// call (57 us with it). Forward-mode tangents and functorch transforms go to the autograd function as well: it has no rule
+/// for them and says so.
 bool differentiated(std::initializer_list<const torch::Tensor*> inputs)
 {
-    if (!at::GradMode::is_enabled()) return false;
+    if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
+    const bool recording = at::GradMode::is_enabled();
     for (const torch::Tensor* t : inputs)
-        if (t->requires_grad()) return true;
+        if ((recording && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined()) return true;
     return false;
 }
 
@@ -176,7 +179,10 @@ public:
     static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor input, torch::Tensor weight, int64_t op, int64_t merge,
                                  int64_t padding, double padding_value, bool save_indices, double noise_scale, int64_t flags)
     {
-        const MorphoCall call = run_morpho_forward(input, weight, op, merge, padding, padding_value, save_indices, noise_scale, flags);
+        MorphoCall call = run_morpho_forward(input, weight, op, merge, padding, padding_value, save_indices, noise_scale, flags);
+        // Erosion's structuring element is saved as a copy (the reference saves the flipped one), so that a program may go on
+        // to change the parameter in place before the backward pass.
+        if ((flags & MC_FLAG_FLIPPED_WEIGHT) != 0 && call.weight4d.is_alias_of(weight)) call.weight4d = call.weight4d.clone();
         ctx->save_for_backward({call.input4d, call.weight4d, call.indices, call.sample_weight});
         ctx->saved_data["op"] = op;
         ctx->saved_data["merge"] = merge;
@@ -417,15 +423,22 @@ SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& w
 }
 
 /// Gradient of the structuring element as the user holds it, from that of w~; adds to the alpha gradient what flows through
-/// w~. Returns `grad` itself where the call had no re-parametrisation.
+/// w~ (meaningless where `raw_weight` is not the structuring element, see save_raw_weight).
 torch::Tensor through_reparametrisation(const mc_desc& d, const torch::Tensor& raw_weight, const torch::Tensor& alphas, const torch::Tensor& grad,
                                         torch::Tensor& grad_alpha_pairs, cudaStream_t stream)
 {
-    if (!raw_weight.defined()) return grad;
     torch::Tensor out = at::empty_like(grad);
     check_status(mc_smorph_reparametrise_backward(&d, raw_weight.data_ptr(), alphas.data_ptr(), grad.data_ptr(), out.data_ptr(),
                                                   grad_alpha_pairs.data_ptr(), stream));
     return out;
+}
+
+/// The structuring element before the re-parametrisation is needed by the alpha gradient alone. Where alpha has none it is
+/// not saved, so that a program may change it in place before the backward pass; backward() then hands w~ in its place and
+/// drops the alpha gradient.
+torch::Tensor save_raw_weight(const torch::Tensor& raw_weight, const torch::Tensor& alpha)
+{
+    return alpha.requires_grad() ? raw_weight : torch::Tensor();
 }
 
 class SmorphFunction : public torch::autograd::Function<SmorphFunction>
@@ -436,7 +449,8 @@ public:
     {
         const SmorphCall call = run_smorph_forward(input, weight, alpha, merge, reparametrise);
         // The backward pass reads the 4-D output: the merge target of MAX and MIN.
-        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d, call.alphas, call.raw_weight});
+        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d, call.alphas, save_raw_weight(call.raw_weight, alpha)});
+        ctx->saved_data["reparametrised"] = reparametrise;
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
@@ -473,7 +487,8 @@ public:
         check_status(mc_smorph_backward(&d, input.data_ptr(), weight.data_ptr(), alphas.data_ptr(), output.data_ptr(), grad_output.data_ptr(),
                                         grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
                                         workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, stream));
-        grad_weight = through_reparametrisation(d, raw_weight, alphas, grad_weight, grad_alpha_pairs, stream);
+        if (ctx->saved_data["reparametrised"].toBool())
+            grad_weight = through_reparametrisation(d, raw_weight.defined() ? raw_weight : weight, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph.cpp:96-98).
         torch::Tensor grad_alpha =
@@ -539,7 +554,8 @@ public:
     {
         const SmorphScmCall call = run_smorph_scm_forward(input, weight, alpha, beta, reparametrise);
         // The backward pass reads the 4-D output: the final value of the soft merge.
-        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d, call.alphas, call.raw_weight});
+        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d, call.alphas, save_raw_weight(call.raw_weight, alpha)});
+        ctx->saved_data["reparametrised"] = reparametrise;
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
         return output_to_original(call.output, input.dim());
@@ -574,7 +590,8 @@ public:
         check_status(mc_smorph_scm_backward(&d, input.data_ptr(), weight.data_ptr(), alphas.data_ptr(), beta.data_ptr(), output.data_ptr(),
                                             grad_output.data_ptr(), grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
                                             grad_beta.data_ptr(), workspace.data_ptr(), ws_bytes, stream));
-        grad_weight = through_reparametrisation(d, raw_weight, alphas, grad_weight, grad_alpha_pairs, stream);
+        if (ctx->saved_data["reparametrised"].toBool())
+            grad_weight = through_reparametrisation(d, raw_weight.defined() ? raw_weight : weight, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph_scm.cpp:81-83).
         torch::Tensor grad_alpha =

@@ -399,3 +399,42 @@ def test_smorph_reparametrisation_kernel(F, shape, k):
         assert p.shape == q.shape and (p - q).abs().max() <= 1e-11 * q.abs().max().clamp_min(1.0)
     with torch.no_grad():
         assert torch.equal(F.smorph(x, w, a, beta, merge), y)
+
+
+def test_parameters_may_change_in_place_before_the_backward_pass(F):
+    """Erosion differentiates with the structuring element of the call, and so does smorph where alpha has no gradient (with
+    one, autograd refuses the call): changing the parameter in place between the two passes is allowed and changes nothing."""
+    torch.manual_seed(5)
+    x = torch.rand(2, 3, 20, 33, device="cuda")
+    for merge in ("sum", "max"):
+        w = (0.1 * torch.randn(4, 3, 3, 3, device="cuda")).requires_grad_(True)
+        want = torch.autograd.grad(F.erosion(x, w, merge).square().sum(), w)[0]
+        y = F.erosion(x, w, merge).square().sum()
+        with torch.no_grad():
+            w.mul_(-2.0)
+        assert torch.allclose(torch.autograd.grad(y, w)[0], want, rtol=1e-4, atol=1e-4 * want.abs().max().item())
+    w = (0.1 * torch.randn(4, 3, 3, 3, device="cuda")).requires_grad_(True)
+    alpha = torch.full((4, 3), 0.7, device="cuda")
+    want = torch.autograd.grad(F.smorph(x, w, alpha).square().sum(), w)[0]
+    y = F.smorph(x, w, alpha).square().sum()
+    with torch.no_grad():
+        w.mul_(-2.0)
+    assert torch.allclose(torch.autograd.grad(y, w)[0], want, rtol=1e-4, atol=1e-4 * want.abs().max().item())
+    y = F.smorph(x, w, alpha.clone().requires_grad_(True)).square().sum()
+    with torch.no_grad():
+        w.mul_(-2.0)
+    with pytest.raises(RuntimeError, match="inplace"):
+        y.backward()
+
+
+def test_tangents_are_refused_and_vmap_runs_slice_by_slice(F):
+    """Forward-mode tangents have no rule here: they raise instead of being dropped on the way. vmap falls back to one call per
+    slice."""
+    import torch.autograd.forward_ad as fwad
+    x, w = torch.rand(2, 3, 20, 33, device="cuda"), torch.randn(4, 3, 3, 3, device="cuda")
+    alpha = torch.ones(4, 3, device="cuda")
+    calls = (lambda t: F.dilation(t, w, "max"), lambda t: F.erosion(t, w), lambda t: F.smorph(t, w, alpha), lambda t: F.sigma_layer(t, w, alpha))
+    for call in calls:
+        with pytest.raises(RuntimeError), fwad.dual_level():
+            call(fwad.make_dual(x, torch.ones_like(x)))
+        assert torch.allclose(torch.func.vmap(call)(x[:, None]), call(x)[:, None], rtol=1e-5, atol=1e-5)
