@@ -13,6 +13,7 @@
 // negated structuring element, x + (-w) being the same IEEE operation as x - w.
 #pragma once
 #include "common.cuh"
+#include "shares.cuh"
 #include "tma.cuh"
 
 namespace mc
@@ -660,7 +661,8 @@ constexpr int FIND_TILE = 16;
 /// one-pixel-per-thread scan above reads 25 (5 x 5) scattered elements of a different channel plane per lane: at 64
 /// channels that is an L2 gather of a few hundred bytes per output pixel and takes half as long as the whole
 /// forward pass. Here a CTA owns (batch element, 16 x 16 tile), stages the windows of a group of input channels
-/// (as many as fit in shared memory; every channel for 64 of them at 5 x 5) and then walks ALL output channels:
+/// (as many as fit in shared memory; every channel for 64 of them at 5 x 5) and then walks the output channels (all of them, or
+/// its share where the tiles are too few for the SMs):
 /// a thread looks up its pixel's winning channel and scans that channel's window in shared memory, with the
 /// output channel's structuring elements staged beside it. The input is read from global memory once per group
 /// (plus the halo), the indices once, and every scan is the reference's strict comparison in kh-major, kw order.
@@ -677,6 +679,7 @@ __global__ void __launch_bounds__(FIND_TILE * FIND_TILE) morpho_find_tap_tiled_k
     const int tiles_x = (g.W + FIND_TILE - 1) / FIND_TILE;
     const int tile_h0 = (blockIdx.x / tiles_x) * FIND_TILE, tile_w0 = (blockIdx.x % tiles_x) * FIND_TILE;
     const int b = blockIdx.y;
+    const int o_begin = share_begin(g.Co, blockIdx.z, gridDim.z), o_end = share_begin(g.Co, blockIdx.z + 1, gridDim.z);
     const int tx = threadIdx.x % FIND_TILE, ty = threadIdx.x / FIND_TILE;
     const int h = tile_h0 + ty, w = tile_w0 + tx;
     const bool live = h < g.H && w < g.W;
@@ -700,17 +703,15 @@ __global__ void __launch_bounds__(FIND_TILE * FIND_TILE) morpho_find_tap_tiled_k
         }
         cp_async_wait_all();
         const int64_t at0 = ((static_cast<int64_t>(b) * g.Co) * g.H + h) * g.W + w;
-        int next = live ? a.idx[at0] : 0;   // the winner of the next output channel is fetched one iteration ahead
-        for (int o = 0; o < g.Co; o++)
+        int next = live ? a.idx[at0 + static_cast<int64_t>(o_begin) * plane] : 0;   // the winner of the next output channel is fetched one iteration ahead
+        for (int o = o_begin; o < o_end; o++)
         {
             __syncthreads();   // windows landed (first pass); the previous output channel's structuring elements are no longer read
-            for (int e = threadIdx.x; e < cc * TAPS; e += NT)
-            {
-                const int c = e / TAPS;
-                sw[e] = __ldg(wb + (static_cast<int64_t>(o) * g.Ci + c0 + c) * TAPS + g.stored_tap(e - c * TAPS));
-            }
+            // A reversed structuring element: the whole group is reversed, its channels with its taps (no division here).
+            const T* wo = wb + (static_cast<int64_t>(o) * g.Ci + c0) * TAPS;
+            for (int e = threadIdx.x; e < cc * TAPS; e += NT) sw[g.flipped ? cc * TAPS - 1 - e : e] = __ldg(wo + e);
             const int packed = next;
-            if (live && o + 1 < g.Co) next = a.idx[at0 + static_cast<int64_t>(o + 1) * plane];
+            if (live && o + 1 < o_end) next = a.idx[at0 + static_cast<int64_t>(o + 1) * plane];
             __syncthreads();
             if (!live) continue;
             const int64_t at = at0 + static_cast<int64_t>(o) * plane;
@@ -718,7 +719,7 @@ __global__ void __launch_bounds__(FIND_TILE * FIND_TILE) morpho_find_tap_tiled_k
             ch = min(max(ch, 0), g.Ci - 1);
             if (ch < c0 || ch >= c0 + cc) continue;
             const T* win = sx + (ch - c0) * (WIN * WIN) + ty * WIN + tx;
-            const T* wk = sw + (ch - c0) * TAPS;
+            const T* wk = sw + (g.flipped ? cc - 1 - (ch - c0) : ch - c0) * TAPS;
             T best = op_init;
             int arg = 0;
 #pragma unroll
@@ -752,7 +753,7 @@ inline bool plan_forward(const Geometry& g, int ob, int stages, ForwardPlan<T>& 
 {
     const size_t window = static_cast<size_t>(g.window_elems()) * sizeof(T), weights = static_cast<size_t>(g.taps()) * ob * sizeof(T);
     const size_t per_channel = stages * (window + weights);
-    const size_t fixed = 128 + stages * (128 + 16);
+    const size_t fixed = 128 + stages * 128 + (stages > 1 ? stages * 16 : 0);   // rounding up between the parts
     if (per_channel + fixed > MAX_SHARED_BYTES) return false;
     const int channels = g.identity ? 1 : g.Ci;
     int chunk = static_cast<int>((96 * 1024 - fixed) / per_channel);
@@ -831,7 +832,10 @@ int launch_forward(const mc_desc& d, const T* x, const T* w, T* y, int32_t* idx,
         auto tiled = morpho_find_tap_tiled_kernel<T, IS_MIN, KW>;
         if (group >= 8 && d.B <= 65535 && tiles <= 0x7fffffffLL && allow_shared(tiled, group * PER_CHANNEL))
         {
-            tiled<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(d.B)), FIND_TILE * FIND_TILE, group * PER_CHANNEL, stream>>>(a, group);
+            // Staging the windows costs a block about as much as six output channels.
+            const int per_sm = static_cast<int>(std::min<size_t>(8, MAX_SHARED_BYTES / (group * PER_CHANNEL + 1024)));
+            const int shares = channel_shares(tiles * d.B, d.Co, per_sm, 6);
+            tiled<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(d.B), static_cast<unsigned>(shares)), FIND_TILE * FIND_TILE, group * PER_CHANNEL, stream>>>(a, group);
             return check_launch("morpho_find_tap_tiled_kernel");
         }
     }

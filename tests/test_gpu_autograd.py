@@ -438,3 +438,19 @@ def test_tangents_are_refused_and_vmap_runs_slice_by_slice(F):
         with pytest.raises(RuntimeError), fwad.dual_level():
             call(fwad.make_dual(x, torch.ones_like(x)))
         assert torch.allclose(torch.func.vmap(call)(x[:, None]), call(x)[:, None], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("k", [3, 5])
+def test_winner_search_of_a_reversed_structuring_element(F, k):
+    """The tap search stages the structuring elements of a group of channels reversed as a whole; with 70 channels there are
+    several groups in double. Whole-number output gradients: weight gradients are exact and equal those of the flipped copy."""
+    torch.manual_seed(6)
+    x = torch.randn(1, 70, 19, 37, dtype=torch.float64, device="cuda")
+    w = torch.randn(3, 70, k, k, dtype=torch.float64, device="cuda")
+    gy = torch.randint(-3, 4, (1, 3, 19, 37), device="cuda").double()
+    got = [t.clone().requires_grad_(True) for t in (x, w)]
+    want = [t.clone().requires_grad_(True) for t in (x, w)]
+    F.erosion(*got, "max", "replicate").backward(gy)
+    torch.ops.morphocore.erosion(want[0], want[1].flip((-2, -1)), 0, 3, 0.0, True, 0.0).backward(gy)
+    for a, b in zip(got, want):
+        assert torch.equal(a.grad, b.grad)
