@@ -43,13 +43,35 @@ struct ScatterBackwardArgs
     T sign;           // +1 dilation, -1 erosion
 };
 
+/// Row and column of a pixel, advanced by a fixed number of pixels without a division.
+struct Pixel
+{
+    struct Step
+    {
+        int h, w;
+        __device__ Step(int n, int W) : h(n / W), w(n - n / W * W) {}
+    };
+    int h, w;
+    __device__ Pixel(int64_t p, int W) : h(static_cast<int>(p / W)), w(static_cast<int>(p - p / W * W)) {}
+    __device__ __forceinline__ void advance(const Step& s, int W)
+    {
+        h += s.h;
+        w += s.w;
+        if (w >= W)
+        {
+            w -= W;
+            h++;
+        }
+    }
+};
+
 /// Backward of the MAX / MIN merges from the packed winners, (channel << 16) | tap: every output pixel sends its
 /// gradient to ONE input pixel and ONE weight bin. HBM-bound work (gy and idx read once, grad_input touched once per
 /// output pixel), so the kernel is shaped for memory parallelism:
 ///   - one CTA per (batch element, output channel, strip of the plane): B * Co * strips CTAs, every SM busy whatever
 ///     the batch; its Ci * taps weight bins live in shared memory until one flush;
 ///   - a thread takes four consecutive pixels per step with 128-bit loads of gy and idx, two steps in flight;
-///   - the four pixels share one row, so the pixel's (h, w) costs one division per step, and K is a compile-time
+///   - the four pixels share one row, so the pixel's (h, w) is advanced once per step, without a division, and K is a compile-time
 ///     constant for the specialised widths, so the tap's (kh, kw) costs none.
 /// A winning tap that read padding adds to grad_weight but not to grad_input, as in the reference
 /// (morphocore/functional/csrc/cpp/morpho_op_cpu_backward.hxx:39-41, 78-84).
@@ -112,30 +134,41 @@ __global__ void __launch_bounds__(THREADS) morpho_backward_scatter_kernel(const 
                 iv = make_int4(0, 0, 0, 0);
             }
         };
+        Pixel at(p_begin + 4 * threadIdx.x, g.W);
+        const Pixel::Step step(STEP, g.W);
         for (int64_t p = p_begin + 4 * threadIdx.x; p < p_end; p += 2 * STEP)
         {
             T g0[4], g1[4];
             int4 i0, i1;
             load(p, g0, i0);
-            load(p + STEP, g1, i1);
-            {
-                const int h = static_cast<int>(p / g.W), w = static_cast<int>(p - static_cast<int64_t>(h) * g.W);
-                route(g0[0], i0.x, h, w); route(g0[1], i0.y, h, w + 1); route(g0[2], i0.z, h, w + 2); route(g0[3], i0.w, h, w + 3);
-            }
-            if (p + STEP < p_end)
-            {
-                const int64_t q = p + STEP;
-                const int h = static_cast<int>(q / g.W), w = static_cast<int>(q - static_cast<int64_t>(h) * g.W);
-                route(g1[0], i1.x, h, w); route(g1[1], i1.y, h, w + 1); route(g1[2], i1.z, h, w + 2); route(g1[3], i1.w, h, w + 3);
-            }
+            load(p + STEP, g1, i1);   // zeros past the end of the strip, which are not routed
+            route(g0[0], i0.x, at.h, at.w); route(g0[1], i0.y, at.h, at.w + 1); route(g0[2], i0.z, at.h, at.w + 2); route(g0[3], i0.w, at.h, at.w + 3);
+            at.advance(step, g.W);
+            route(g1[0], i1.x, at.h, at.w); route(g1[1], i1.y, at.h, at.w + 1); route(g1[2], i1.z, at.h, at.w + 2); route(g1[3], i1.w, at.h, at.w + 3);
+            at.advance(step, g.W);
         }
     }
     else
     {
-        for (int64_t p = p_begin + threadIdx.x; p < p_end; p += THREADS)
+        Pixel at(p_begin + threadIdx.x, g.W);
+        const Pixel::Step step(THREADS, g.W);
+        for (int64_t p = p_begin + threadIdx.x; p < p_end; p += 4 * THREADS)
         {
-            const int h = static_cast<int>(p / g.W);
-            route(__ldg(gyp + p), __ldg(ip + p), h, static_cast<int>(p - static_cast<int64_t>(h) * g.W));
+            T grad[4];
+            int32_t winner[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+                const bool in = p + i * THREADS < p_end;
+                grad[i] = in ? __ldg(gyp + p + i * THREADS) : T(0);
+                winner[i] = in ? __ldg(ip + p + i * THREADS) : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+                route(grad[i], winner[i], at.h, at.w);
+                at.advance(step, g.W);
+            }
         }
     }
     if (a.copies == 0) return;
@@ -143,7 +176,8 @@ __global__ void __launch_bounds__(THREADS) morpho_backward_scatter_kernel(const 
     for (int e = threadIdx.x; e < nbins; e += THREADS)
     {
         T sum = T(0);
-        for (int c = 0; c < a.copies; c++) sum += bins[e * a.copies + c];
+        // Each thread starts at a copy of its own: the 32 / copies bins whose copies share the banks are read one bank apart.
+        for (int c = 0; c < a.copies; c++) sum += bins[e * a.copies + ((c + (e * a.copies >> 5)) & (a.copies - 1))];
         if (sum != T(0)) atomic_add(gwo + e / taps * taps + g.stored_tap(e % taps), a.sign * sum);
     }
 }
