@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "shares.cuh"
 #include "morpho_forward.cuh"
 
 namespace mc
@@ -264,8 +265,8 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_kernel(const
     for (int e = threadIdx.x; e < g.window_elems(); e += THREADS) sg[e] = T(0);
     for (int e = threadIdx.x; e < OB * taps * a.copies; e += THREADS) bins[e] = T(0);
 
-    const int o_begin = g.identity ? ci : 0;
-    const int o_end = g.identity ? ci + 1 : g.Co;
+    const int o_begin = g.identity ? ci : share_begin(g.Co, blockIdx.y, gridDim.y);
+    const int o_end = g.identity ? ci + 1 : share_begin(g.Co, blockIdx.y + 1, gridDim.y);
     for (int o0 = o_begin; o0 < o_end; o0 += OB)
     {
         __syncthreads();
@@ -646,30 +647,35 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     a.scale = d.merge == MC_MERGE_AVERAGE ? T(1.0) / static_cast<T>(d.Ci) : T(1.0);
     a.sign = d.op == MC_OP_DILATION ? T(1) : T(-1);
     const size_t taps = static_cast<size_t>(d.kH) * d.kW;
-    const int64_t blocks = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
-    if (blocks > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
+    const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
+    if (items > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
+    // CTAs that divide the output channels of a tile (grid.y); staging its window and adding up grad_input cost one about as
+    // much as four of them.
+    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, 2, 4);
+    const dim3 blocks(static_cast<unsigned>(items), static_cast<unsigned>(shares));
+    const int channels = a.g.identity ? 1 : (d.Co + shares - 1) / shares;   // the most a CTA walks
     if constexpr (sizeof(T) == 4 && (KW == 3 || KW == 5))
     {
-        const size_t bytes = pairs_regs_smem<KW>(a.g, a.g.identity ? 1 : d.Co);
+        const size_t bytes = pairs_regs_smem<KW>(a.g, channels);
         if (bytes > 0)
         {
             auto fast = morpho_backward_pairs_regs_kernel<IS_MIN, KW>;
             if (allow_shared(fast, bytes))
             {
-                fast<<<static_cast<unsigned>(blocks), THREADS, bytes, stream>>>(a);
+                fast<<<blocks, THREADS, bytes, stream>>>(a);
                 return check_launch("morpho_backward_pairs_regs_kernel");
             }
         }
     }
     if constexpr (sizeof(T) == 4 && (KW == 3 || KW == 5 || KW == 7))
     {
-        const size_t bytes = pairs_rows_smem<KW>(a.g, a.g.identity ? 1 : d.Co);
+        const size_t bytes = pairs_rows_smem<KW>(a.g, channels);
         if (bytes > 0)
         {
             auto fast = morpho_backward_pairs_rows_kernel<IS_MIN, KW>;
             if (allow_shared(fast, bytes))
             {
-                fast<<<static_cast<unsigned>(blocks), THREADS, bytes, stream>>>(a);
+                fast<<<blocks, THREADS, bytes, stream>>>(a);
                 return check_launch("morpho_backward_pairs_rows_kernel");
             }
         }
@@ -702,7 +708,7 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     const size_t smem = fixed + taps * OB * a.copies * sizeof(T);
     auto kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB>;
     if (!allow_shared(kernel, smem)) { set_last_error("cannot opt in to %zu bytes of shared memory", smem); return MC_ERR_UNSUPPORTED; }
-    kernel<<<static_cast<unsigned>(blocks), THREADS, smem, stream>>>(a);
+    kernel<<<blocks, THREADS, smem, stream>>>(a);
     return check_launch("morpho_backward_pairs_kernel");
 }
 

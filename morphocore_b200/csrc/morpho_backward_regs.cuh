@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_regs_kernel(
     const int64_t plane = g.plane();
     const int wci = g.identity ? 1 : g.Ci;
     const int wi = g.identity ? 0 : ci;
-    const int o_begin = g.identity ? ci : 0;
-    const int o_end = g.identity ? ci + 1 : g.Co;
+    const int o_begin = g.identity ? ci : share_begin(g.Co, blockIdx.y, gridDim.y);
+    const int o_end = g.identity ? ci + 1 : share_begin(g.Co, blockIdx.y + 1, gridDim.y);
     const int channels = o_end - o_begin;
 
     T* foot = reinterpret_cast<T*>(smem_raw);                                      // [WARPS][FR * FC][32]; first the staged window

@@ -46,8 +46,8 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_rows_kernel(
     const int wci = g.identity ? 1 : g.Ci;
     const int wi = g.identity ? 0 : ci;
     const T op_init = IS_MIN ? Limits<T>::inf() : -Limits<T>::inf();
-    const int o_begin = g.identity ? ci : 0;
-    const int o_end = g.identity ? ci + 1 : g.Co;
+    const int o_begin = g.identity ? ci : share_begin(g.Co, blockIdx.y, gridDim.y);
+    const int o_end = g.identity ? ci + 1 : share_begin(g.Co, blockIdx.y + 1, gridDim.y);
     const int o_span = (o_end - o_begin + OB - 1) / OB * OB;
 
     load_window(sx, a.x + (static_cast<int64_t>(b) * g.Ci + ci) * plane, g, tile_h0, tile_w0, a.fill);

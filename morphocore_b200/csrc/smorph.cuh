@@ -17,6 +17,8 @@
 
 #include "common.cuh"
 #include "morpho_backward.cuh"
+#include "clusters.cuh"
+#include "shares.cuh"
 #include "tma.cuh"
 
 namespace mc
@@ -752,6 +754,7 @@ struct SmorphForwardArgs
     int o_groups;
     int chunk;
     int factorise;    // use the factorised path where it is safe (merges without winner test)
+    int cluster;      // CTAs that divide the input channels of one tile and group of output channels
     unsigned int* errors;  // counter of timed-out waits
     uint64_t wait_limit_ns; // bound of one wait on a TMA copy
 };
@@ -790,9 +793,10 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     const bool factorise = FACTOR && a.factorise != 0;
 
     const int tiles = g.tiles_x * g.tiles_y;
-    const int og = blockIdx.x % a.o_groups;
-    const int tile = (blockIdx.x / a.o_groups) % tiles;
-    const int b = blockIdx.x / (a.o_groups * tiles);
+    const int rank = blockIdx.x % a.cluster, item = blockIdx.x / a.cluster;
+    const int og = item % a.o_groups;
+    const int tile = (item / a.o_groups) % tiles;
+    const int b = item / (a.o_groups * tiles);
     const int tile_h0 = (tile / g.tiles_x) * TILE_H, tile_w0 = (tile % g.tiles_x) * TILE_W;
     int tx, ty, half;
     bool warp_live, split;
@@ -804,13 +808,14 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     const int o0 = og * OB;
     const int64_t plane = g.plane();
     const T* xb = a.x + static_cast<int64_t>(b) * g.Ci * plane;
-    const int channels = g.identity ? 1 : g.Ci;
     const int wci = g.identity ? 1 : g.Ci;
     const int first_channel = g.identity ? o0 : 0;
+    // Input channels of this CTA: all of them, or its part where the CTAs of a cluster divide them.
+    const int c_begin = g.identity ? 0 : share_begin(g.Ci, rank, a.cluster), c_end = g.identity ? 1 : share_begin(g.Ci, rank + 1, a.cluster);
 
     // Signs of every pair of this CTA: a single sign needs one window per channel, both signs need two.
     bool any_pos = false, any_neg = false;
-    for (int e = threadIdx.x; e < channels * OB; e += THREADS)
+    for (int e = c_begin * OB + threadIdx.x; e < c_end * OB; e += THREADS)
     {
         const int o = e % OB, c = e / OB;
         if (o0 + o >= g.Co) continue;
@@ -845,10 +850,10 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     auto issue = [&](int n) {
         uint64_t* bar = full + (n & 1);
         T* stage = sx0 + (n & 1) * 2 * slot_elems;
-        const int c_first = first_channel + n * span;
+        const int c_first = first_channel + c_begin + n * span;
         // The second copy brings the same channels again (other border fill) or the next `chunk` channels; a
         // copy that starts past the last channel is skipped.
-        const bool second = mixed || (n * span + a.chunk < channels);
+        const bool second = mixed || (c_begin + n * span + a.chunk < c_end);
         mbar_expect_tx(bar, second ? 2 * slot_bytes : slot_bytes);
         tma_load_4d(stage, &tmap, bar, tile_w0 - g.halo_left(), tile_h0 - g.halo_top(), c_first, b);
         if (second) tma_load_4d(stage + slot_elems, &tmap, bar, tile_w0 - g.halo_left(), tile_h0 - g.halo_top(), mixed ? c_first : c_first + a.chunk, b);
@@ -907,14 +912,15 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
         return stage + (c >= a.chunk ? slot_elems + (c - a.chunk) * welems : c * welems);
     };
     int n = 0;
-    for (int c0 = 0; c0 < channels; c0 += span, n++)
+    bool failed = false;
+    for (int c0 = c_begin; c0 < c_end; c0 += span, n++)
     {
-        const int cc = min(span, channels - c0);
+        const int cc = min(span, c_end - c0);
         T* stage = sx0 + (USE_TMA ? (n & 1) * 2 * slot_elems : 0);
         __syncthreads();
         if constexpr (USE_TMA)
         {
-            if (threadIdx.x == 0 && c0 + span < channels)
+            if (threadIdx.x == 0 && c0 + span < c_end)
             {
                 fence_async_smem();
                 issue(n + 1);
@@ -994,7 +1000,8 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
             if (!mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns))
             {
                 if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
-                return;  // every thread of the CTA waits on the same barrier and gives up together
+                failed = true;   // every thread of the CTA waits on the same barrier and gives up together
+                break;           // (the other CTAs of its cluster still wait for it below)
             }
             if (border)
             {
@@ -1109,45 +1116,117 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
 
     const T divisor = static_cast<T>(g.Ci);
     T* dst = STATS ? a.counts : a.y;
+    // One pixel of the result: the merged value, for the smooth merge with the extremum and the sum of its weights.
+    auto store = [&](int o, int rr, int j, T v, T extremum, T sum) {
+        const int h = tile_h0 + ty * PATCH_H + rr, w = tile_w0 + tx * PATCH_W + j;
+        if (o >= o_count || !warp_live || o0 + o_base + o >= g.Co || h >= g.H || w >= g.W) return;
+        const int64_t at = ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w;
+        if constexpr (SOFT)
+        {
+            const T inv = T(1) / sum;
+            if (a.soft_ref != nullptr)
+            {
+                a.soft_ref[at] = extremum;
+                a.soft_inv[at] = inv;
+            }
+            else a.y[at] = v * inv;
+        }
+        else
+        {
+            if (!STATS && a.merge == MC_MERGE_AVERAGE) v = v / divisor;
+            dst[at] = v;
+        }
+    };
+    if (a.cluster == 1)
+    {
+        if (failed) return;
+#pragma unroll
+        for (int o = 0; o < OB; o++)
+#pragma unroll
+            for (int rr = 0; rr < PATCH_H; rr++)
+#pragma unroll
+                for (int j = 0; j < PATCH_W; j++)
+                {
+                    if constexpr (SOFT) store(o, rr, j, merged[o][rr][j], soft_sign[o] * soft_m[o][rr][j], soft_s[o][rr][j]);
+                    else store(o, rr, j, FACTOR ? merged[o][rr][j] + offset[o] : merged[o][rr][j], T(0), T(0));
+                }
+        return;
+    }
+    // Every CTA of the cluster leaves its part in the place of its windows; rank r merges and stores the pixels r, r + cluster,
+    // ... of every thread, in the order of the ranks.
+    constexpr int PIXELS = OB * PATCH_H * PATCH_W;
+    __syncthreads();   // the windows are no longer read
+    T* slots = sx0 + threadIdx.x;   // [PIXELS][THREADS] merged values; then the offsets [OB], or extrema and sums [PIXELS] each
 #pragma unroll
     for (int o = 0; o < OB; o++)
+    {
 #pragma unroll
-        for (int rr = 0; rr < PATCH_H; rr++)
-#pragma unroll
-            for (int j = 0; j < PATCH_W; j++)
+        for (int p = 0; p < PATCH_H * PATCH_W; p++)
+        {
+            const int at = (o * PATCH_H * PATCH_W + p) * THREADS, rr = p / PATCH_W, j = p % PATCH_W;
+            slots[at] = merged[o][rr][j];
+            if constexpr (SOFT)
             {
-                const int h = tile_h0 + ty * PATCH_H + rr, w = tile_w0 + tx * PATCH_W + j;
-                if (o >= o_count || !warp_live || o0 + o_base + o >= g.Co || h >= g.H || w >= g.W) continue;
-                T v = merged[o][rr][j];
-                const int64_t at = ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w;
-                if constexpr (SOFT)
-                {
-                    const T inv = T(1) / soft_s[o][rr][j];
-                    if (a.soft_ref != nullptr)
-                    {
-                        a.soft_ref[at] = soft_sign[o] * soft_m[o][rr][j];
-                        a.soft_inv[at] = inv;
-                    }
-                    else a.y[at] = v * inv;
-                    continue;
-                }
-                if constexpr (FACTOR) v += offset[o];
-                if (!STATS && a.merge == MC_MERGE_AVERAGE) v = v / divisor;
-                dst[at] = v;
+                slots[PIXELS * THREADS + at] = soft_m[o][rr][j];
+                slots[2 * PIXELS * THREADS + at] = soft_s[o][rr][j];
             }
+        }
+        if constexpr (!SOFT) slots[(PIXELS + o) * THREADS] = offset[o];
+    }
+    cluster_sync();
+    if (!failed)
+    {
+        const uint32_t mine = smem_addr(slots);
+        auto part = [&](int at, int r) { return load_cluster<T>(mine + at * THREADS * static_cast<int>(sizeof(T)), r); };
+        for (int i = rank; i < PIXELS; i += a.cluster)
+        {
+            const int o = i / (PATCH_H * PATCH_W), rr = i / PATCH_W % PATCH_H, j = i % PATCH_W;
+            T v = part(i, 0);
+            if constexpr (SOFT)
+            {
+                const T bt = o0 + o_base + o < g.Co ? __ldg(a.beta + o0 + o_base + o) : T(0);
+                const T sign = bt >= T(0) ? T(1) : T(-1), scale = exp_scale(bt >= T(0) ? bt : -bt);
+                T top = part(PIXELS + i, 0), sum = part(2 * PIXELS + i, 0);
+                for (int r = 1; r < a.cluster; r++)
+                {
+                    const T other = part(PIXELS + i, r), higher = top < other ? other : top;
+                    const T keep = soft_exp(top - higher, scale), add = soft_exp(other - higher, scale);
+                    v = fma(v, keep, add * part(i, r));
+                    sum = fma(sum, keep, add * part(2 * PIXELS + i, r));
+                    top = higher;
+                }
+                store(o, rr, j, v, sign * top, sum);
+            }
+            else
+            {
+                T off = part(PIXELS + o, 0);
+                for (int r = 1; r < a.cluster; r++)
+                {
+                    const T other = part(i, r);
+                    if (!STATS && a.merge == MC_MERGE_MAX) v = v < other ? other : v;
+                    else if (!STATS && a.merge == MC_MERGE_MIN) v = other < v ? other : v;
+                    else v += other;
+                    off += part(PIXELS + o, r);
+                }
+                store(o, rr, j, FACTOR ? v + off : v, T(0), T(0));
+            }
+        }
+    }
+    cluster_sync();   // nobody leaves while its part is read
 }
 
 template <typename T, int KW, int OB, int MODE, bool USE_TMA>
 int launch_smorph_forward_variant(const SmorphForwardArgs<T>& a, const CUtensorMap& tmap, int64_t blocks, size_t smem, cudaStream_t stream)
 {
     auto kernel = smorph_forward_kernel<T, KW, OB, MODE, USE_TMA>;
+    if (a.cluster > 1)   // the parts of a cluster's CTA
+        smem = std::max(smem, 128 + static_cast<size_t>(OB) * (MODE == 2 ? 3 * PATCH_H * PATCH_W : PATCH_H * PATCH_W + 1) * THREADS * sizeof(T));
     if (!allow_shared(kernel, smem))
     {
         set_last_error("cannot opt in to %zu bytes of shared memory", smem);
         return MC_ERR_UNSUPPORTED;
     }
-    kernel<<<static_cast<unsigned>(blocks), THREADS, smem, stream>>>(a, tmap);
-    return check_launch("smorph_forward_kernel");
+    return launch_clusters(kernel, a.cluster, blocks, smem, stream, "smorph_forward_kernel", a, tmap);
 }
 
 template <typename T, int KW, int OB>
@@ -1162,9 +1241,10 @@ int launch_smorph_forward(const mc_desc& d, const T* x, const T* w, const T* alp
     a.o_groups = (d.Co + OB - 1) / OB;
     a.errors = device_error_counter();
     a.wait_limit_ns = wait_limit_ns();
-    const int channels = a.g.identity ? 1 : d.Ci;
     const int64_t blocks = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * a.o_groups * d.B;
     if (blocks > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
+    a.cluster = a.g.identity ? 1 : cluster_size(blocks, d.Ci, sizeof(T) == 8 ? 1 : 2);
+    const int channels = a.g.identity ? 1 : (d.Ci + a.cluster - 1) / a.cluster;   // the most a CTA walks
     // Per channel: two window slots (one per sign) per stage, the structuring elements, signs and scales.
     const size_t window = static_cast<size_t>(a.g.window_elems()) * sizeof(T);
     const bool stats = counts != nullptr;
@@ -1467,7 +1547,10 @@ __device__ __forceinline__ void smorph_taps_backward(const float* __restrict__ w
 /// SOFT: the smooth channel merge (its own instantiation, so that the other merges keep their register allocation).
 /// FAST (3 x 3 float, sum / mean merges, grad_output aligned for cp.async): the channel loop holds nothing but the
 /// staging of the next channel's gradients and the bounded form of the pair, see there.
-template <typename T, int KH, int KW, bool SOFT, bool FAST = false>
+/// SHARED: several CTAs (grid.y) divide the output channels of a tile, see channel_shares. An instantiation of its own for the
+/// specialised float kernels, whose channel loop has no register to spare for the bounds: 57.0 against 58.6 ms over the two
+/// layers of the four-layer model at B = 32.
+template <typename T, int KH, int KW, bool SOFT, bool FAST = false, bool SHARED = true>
 __global__ void __launch_bounds__(THREADS, (sizeof(T) == 8 || KH >= 5) ? 1 : 2) smorph_backward_kernel(const SmorphBackwardArgs<T> a)
 {
     static_assert(!FAST || (sizeof(T) == 4 && KH == 3 && KW == 3 && !SOFT), "the fast loop is the 3 x 3 float kernel's");
@@ -1516,8 +1599,8 @@ __global__ void __launch_bounds__(THREADS, (sizeof(T) == 8 || KH >= 5) ? 1 : 2) 
     const int wci = g.identity ? 1 : g.Ci;
     const int wi = g.identity ? 0 : ci;
     const bool winner_takes_all = a.merge == MC_MERGE_MAX || a.merge == MC_MERGE_MIN;
-    const int o_begin = g.identity ? ci : 0;
-    const int o_end = g.identity ? ci + 1 : g.Co;
+    const int o_begin = g.identity ? ci : (SHARED ? share_begin(g.Co, blockIdx.y, gridDim.y) : 0);
+    const int o_end = g.identity ? ci + 1 : (SHARED ? share_begin(g.Co, blockIdx.y + 1, gridDim.y) : g.Co);
 
     bool has_pos = false, has_neg = false;
     for (int o = o_begin + threadIdx.x; o < o_end; o += THREADS)
@@ -2064,20 +2147,25 @@ int launch_smorph_backward(const mc_desc& d, const T* x, const T* w, const T* al
     // (The 5 x 5 and 7 x 7 float kernels run one CTA per SM anyway: their chunk may take twice that.)
     const size_t budget = fixed + per_o > 100 * 1024 ? MAX_SHARED_BYTES : (a.factorise ? 200 * 1024 : 100 * 1024);
     int chunk = static_cast<int>((budget - fixed) / per_o);
-    chunk = std::max(1, std::min(chunk, a.g.identity ? 1 : d.Co));
+    const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
+    if (items > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
+    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, (sizeof(T) == 8 || KH >= 5) ? 1 : 2, 2);
+    chunk = std::max(1, std::min(chunk, a.g.identity ? 1 : (d.Co + shares - 1) / shares));
     a.o_chunk = chunk;
     const size_t smem = fixed + per_o * chunk;
     a.grad_stage = stage_grad ? static_cast<int>((smem - GRAD_SLOTS) / 16 * 16) : 0;
-    const int64_t blocks = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
-    if (blocks > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
+    const dim3 blocks(static_cast<unsigned>(items), static_cast<unsigned>(shares));
     auto launch = [&](auto kernel) {
         if (!allow_shared(kernel, smem)) { set_last_error("cannot opt in to %zu bytes of shared memory", smem); return static_cast<int>(MC_ERR_UNSUPPORTED); }
-        kernel<<<static_cast<unsigned>(blocks), THREADS, smem, stream>>>(a);
+        kernel<<<blocks, THREADS, smem, stream>>>(a);
         return check_launch("smorph_backward_kernel");
     };
     if (d.merge == MC_MERGE_SMOOTH) return launch(smorph_backward_kernel<T, KH, KW, true>);
     if constexpr (sizeof(T) == 4 && KH == 3 && KW == 3)
-        if (a.bounded && a.grad_async && d.merge != MC_MERGE_MAX && d.merge != MC_MERGE_MIN) return launch(smorph_backward_kernel<T, KH, KW, false, true>);
+        if (a.bounded && a.grad_async && d.merge != MC_MERGE_MAX && d.merge != MC_MERGE_MIN)
+            return shares == 1 ? launch(smorph_backward_kernel<T, KH, KW, false, true, false>) : launch(smorph_backward_kernel<T, KH, KW, false, true>);
+    if constexpr (sizeof(T) == 4 && KH > 0)
+        if (shares == 1) return launch(smorph_backward_kernel<T, KH, KW, false, false, false>);
     return launch(smorph_backward_kernel<T, KH, KW, false>);
 }
 

@@ -24,6 +24,10 @@
 //     window for pairs of the other sign.
 // A pair whose exponent range |alpha| log2(e) (range of x in the block + range of w) exceeds LEAN_RANGE binades takes the
 // max-subtracting evaluation instead (warp-uniform branch: large |alpha|, or inputs spread widely inside one block).
+//
+// A small batch has too few tiles for 148 SMs, or a last wave that is nearly empty: the input channels of a tile are then
+// divided among the CTAs of a cluster (cluster_size), whose partial sums meet in distributed shared memory at the end, in
+// the order of the ranks (the result does not depend on timing).
 #pragma once
 
 namespace mc
@@ -39,6 +43,7 @@ struct LeanForwardArgs
     int merge;
     int o_groups;
     int chunk;               // input channels staged per barrier
+    int cluster;             // CTAs that divide the input channels of one tile and group of output channels
     unsigned int* errors;    // counter of timed-out waits
     uint64_t wait_limit_ns;  // bound of one wait on a TMA copy
 };
@@ -148,7 +153,9 @@ __device__ __forceinline__ void lean_factor_pair(const float4* __restrict__ rows
 template <int KW> constexpr size_t lean_channel_bytes() { return static_cast<size_t>(KW * KW) * LEAN_OB * (sizeof(float2) + sizeof(float)) + LEAN_OB * sizeof(float4); }
 template <int KW> constexpr size_t lean_fixed_bytes() { return 128 + 2 * 128 + 16 + (THREADS / 32) * static_cast<size_t>(LeanTable<KW>::BYTES); }
 
-template <int KW>
+/// CLUSTER: an instantiation of its own, because the kernel has no register to spare for the bounds of its channels (24.9
+/// against 25.6 ms over the two layers of the four-layer model at B = 32).
+template <int KW, bool CLUSTER>
 __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const LeanForwardArgs a, const __grid_constant__ CUtensorMap tmap)
 {
     using L = FactorLayout<KW>;
@@ -170,9 +177,12 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
                   + warp * (Tb::BYTES / 16);                                    // this warp's (E, A) table
 
     const int tiles = g.tiles_x * g.tiles_y;
-    const int og = blockIdx.x % a.o_groups;
-    const int tile = (blockIdx.x / a.o_groups) % tiles;
-    const int b = blockIdx.x / (a.o_groups * tiles);
+    const int cluster = CLUSTER ? a.cluster : 1;
+    const int rank = blockIdx.x % cluster, item = blockIdx.x / cluster;
+    const int og = item % a.o_groups;
+    const int tile = (item / a.o_groups) % tiles;
+    const int b = item / (a.o_groups * tiles);
+    const int c_begin = CLUSTER ? share_begin(g.Ci, rank, cluster) : 0, c_end = CLUSTER ? share_begin(g.Ci, rank + 1, cluster) : g.Ci;
     const int tile_h0 = (tile / g.tiles_x) * TILE_H, tile_w0 = (tile % g.tiles_x) * TILE_W;
     int tx, ty, half;
     bool warp_live, split;
@@ -194,7 +204,7 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
     auto issue = [&](int n) {
         uint64_t* bar = full + (n & 1);
         mbar_expect_tx(bar, stage_bytes);
-        tma_load_4d(sx0 + (n & 1) * stage_elems, &tmap, bar, tile_w0 - g.halo_left(), tile_h0 - g.halo_top(), n * a.chunk, b);
+        tma_load_4d(sx0 + (n & 1) * stage_elems, &tmap, bar, tile_w0 - g.halo_left(), tile_h0 - g.halo_top(), c_begin + n * a.chunk, b);
     };
     if (threadIdx.x == 0) issue(0);
 
@@ -237,12 +247,13 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
     }
 
     int n = 0;
-    for (int c0 = 0; c0 < g.Ci; c0 += a.chunk, n++)
+    bool failed = false;
+    for (int c0 = c_begin; c0 < c_end; c0 += a.chunk, n++)
     {
-        const int cc = min(a.chunk, g.Ci - c0);
+        const int cc = min(a.chunk, c_end - c0);
         const float* stage = sx0 + (n & 1) * stage_elems;
         __syncthreads();   // every warp is done with the other stage's windows and with the tables below
-        if (threadIdx.x == 0 && c0 + a.chunk < g.Ci)
+        if (threadIdx.x == 0 && c0 + a.chunk < c_end)
         {
             fence_async_smem();
             issue(n + 1);
@@ -285,7 +296,9 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
         if (!mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns))
         {
             if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
-            return;  // every thread of the CTA waits on the same barrier and gives up together
+            if constexpr (!CLUSTER) return;
+            failed = true;   // every thread of the CTA waits on the same barrier and gives up together
+            break;           // (the other CTAs of its cluster still wait for it below)
         }
         __syncthreads();
         if (!warp_live) continue;
@@ -398,34 +411,61 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
         }
     }
 
-    if (!warp_live) return;
     const float divisor = static_cast<float>(g.Ci);
     const bool vec_store = (g.W % 4 == 0) && (reinterpret_cast<uintptr_t>(a.y) % 16 == 0);
-#pragma unroll
-    for (int o = 0; o < OB; o++)
-    {
-        if (o >= o_count || o0 + o_base + o >= g.Co) break;
-#pragma unroll
-        for (int rr = 0; rr < PATCH_H; rr++)
+    auto store = [&](int o, int rr, float4 v) {
+        const int h = tile_h0 + ty * PATCH_H + rr, w0 = tile_w0 + tx * PATCH_W;
+        if (!warp_live || o >= o_count || o0 + o_base + o >= g.Co || h >= g.H || w0 >= g.W) return;
+        if (a.merge == MC_MERGE_AVERAGE) v = make_float4(v.x / divisor, v.y / divisor, v.z / divisor, v.w / divisor);
+        float* dst = a.y + ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w0;
+        if (vec_store && w0 + PATCH_W <= g.W) *reinterpret_cast<float4*>(dst) = v;
+        else
         {
-            const int h = tile_h0 + ty * PATCH_H + rr, w0 = tile_w0 + tx * PATCH_W;
-            if (h >= g.H || w0 >= g.W) continue;
-            float out[PATCH_W];
+            const float out[PATCH_W] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int j = 0; j < PATCH_W; j++)
-            {
-                const float v = merged[o][rr][j] + offset[o];
-                out[j] = a.merge == MC_MERGE_AVERAGE ? v / divisor : v;
-            }
-            float* dst = a.y + ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w0;
-            if (vec_store && w0 + PATCH_W <= g.W) *reinterpret_cast<float4*>(dst) = make_float4(out[0], out[1], out[2], out[3]);
-            else
-            {
+                if (w0 + j < g.W) dst[j] = out[j];
+        }
+    };
+    if constexpr (!CLUSTER)
+    {
 #pragma unroll
-                for (int j = 0; j < PATCH_W; j++)
-                    if (w0 + j < g.W) dst[j] = out[j];
+        for (int o = 0; o < OB; o++)
+#pragma unroll
+            for (int rr = 0; rr < PATCH_H; rr++)
+                store(o, rr, make_float4(merged[o][rr][0] + offset[o], merged[o][rr][1] + offset[o], merged[o][rr][2] + offset[o], merged[o][rr][3] + offset[o]));
+    }
+    else
+    {
+        // Every CTA leaves its sums in the place of its windows; rank r adds up and stores rows r, r + cluster, ... of the eight
+        // (output channel, patch row) rows of every thread.
+        static_assert(OB == 4 && PATCH_W == 4, "a row of the patch and the offsets of the output channels are one float4 each");
+        __syncthreads();   // the windows and tables are no longer read
+        float4* slots = reinterpret_cast<float4*>(smem_raw + 128) + threadIdx.x;
+#pragma unroll
+        for (int o = 0; o < OB; o++)
+#pragma unroll
+            for (int rr = 0; rr < PATCH_H; rr++)
+                slots[(o * PATCH_H + rr) * THREADS] = make_float4(merged[o][rr][0], merged[o][rr][1], merged[o][rr][2], merged[o][rr][3]);
+        slots[OB * PATCH_H * THREADS] = make_float4(offset[0], offset[1], offset[2], offset[3]);
+        cluster_sync();
+        if (!failed)
+        {
+            const uint32_t mine = smem_addr(slots);
+            for (int i = rank; i < OB * PATCH_H; i += cluster)
+            {
+                float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float off = 0.0f;
+                for (int r = 0; r < cluster; r++)
+                {
+                    const float4 v = load_cluster_float4(mine + i * THREADS * 16, r);
+                    sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+                    off += load_cluster<float>(mine + OB * PATCH_H * THREADS * 16 + (i / PATCH_H) * 4, r);
+                }
+                store(i / PATCH_H, i % PATCH_H, make_float4(sum.x + off, sum.y + off, sum.z + off, sum.w + off));
             }
         }
+        cluster_sync();   // nobody leaves while its sums are read
     }
 }
 
@@ -441,20 +481,21 @@ int launch_smorph_forward_lean(const mc_desc& d, const float* x, const float* w,
     a.o_groups = (d.Co + LEAN_OB - 1) / LEAN_OB;
     a.errors = device_error_counter();
     a.wait_limit_ns = wait_limit_ns();
-    const int64_t blocks = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * a.o_groups * d.B;
-    if (blocks > 0x7fffffffLL) return MC_ERR_UNSUPPORTED;
+    const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * a.o_groups * d.B;
+    if (items > 0x7fffffffLL) return MC_ERR_UNSUPPORTED;
+    a.cluster = cluster_size(items, d.Ci, 2);
     const size_t window = static_cast<size_t>(a.g.window_elems()) * sizeof(float);
     const size_t per_channel = 2 * ((window + 127) / 128 * 128) + lean_channel_bytes<KW>(), fixed = lean_fixed_bytes<KW>();
     int chunk = static_cast<int>((100 * 1024 - fixed) / per_channel);
-    chunk = std::max(1, std::min(std::min(chunk, 8), d.Ci));
-    const size_t smem = fixed + per_channel * chunk + 256;
+    chunk = std::max(1, std::min(std::min(chunk, 8), (d.Ci + a.cluster - 1) / a.cluster));
+    size_t smem = fixed + per_channel * chunk + 256;
+    if (a.cluster > 1) smem = std::max(smem, 128 + (LEAN_OB * PATCH_H + 1) * THREADS * sizeof(float4));   // the sums of a CTA
     CUtensorMap tmap{};
     if (!make_window_tensor_map(&tmap, x, sizeof(float), d.B, d.Ci, d.H, d.W, a.g.win_stride, a.g.win_rows, chunk)) return MC_ERR_UNSUPPORTED;
     a.chunk = chunk;
-    auto kernel = smorph_forward_lean_kernel<KW>;
+    auto kernel = a.cluster > 1 ? smorph_forward_lean_kernel<KW, true> : smorph_forward_lean_kernel<KW, false>;
     if (!allow_shared(kernel, smem)) return MC_ERR_UNSUPPORTED;
-    kernel<<<static_cast<unsigned>(blocks), THREADS, smem, stream>>>(a, tmap);
-    return check_launch("smorph_forward_lean_kernel");
+    return launch_clusters(kernel, a.cluster, items, smem, stream, "smorph_forward_lean_kernel", a, tmap);
 }
 
 /// Double precision has no such kernel: the caller takes the general one.

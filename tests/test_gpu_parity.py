@@ -78,6 +78,26 @@ def test_morph_exhaustive_small_shapes(C, op, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("k", [(3, 3), (5, 5), (4, 6), (1, 7), (9, 9)])
+@pytest.mark.parametrize("W", [33, 61, 64, 99])
+def test_forward_staging_edges(C, k, W, dtype):
+    """Windows and structuring elements travel one chunk of channels ahead: widths TMA can and cannot address, warps of a tile
+    outside the image, one chunk and several with a remainder, output channels that fill a group of the kernel and that do not.
+    Values and winner indices against the oracle, bit for bit."""
+    rng = np.random.default_rng(W * 10 + k[1])
+    for (Ci, Co, H) in ((1, 1, 9), (7, 3, 33), (19, 6, 25)):
+        x = rng.standard_normal((2, Ci, H, W)).astype(dtype)
+        w = (0.3 * rng.standard_normal((Co, Ci, *k))).astype(dtype)
+        for op, merge, padding, pv in (("dilation", "sum", "replicate", 0.0), ("erosion", "max", "constant", 0.5), ("dilation", "min", "geodesic", 0.0)):
+            want, want_idx = O.morpho_forward(op, x, w, merge, padding, pv, with_index=True)
+            got, got_idx = C.morpho_forward(op, dev(x), dev(w), merge, padding, pv, with_index=True)
+            assert np.array_equal(got.cpu().numpy(), want), (op, merge, Ci, Co)
+            if merge != "sum":
+                assert np.array_equal(got_idx.cpu().numpy(), want_idx), (op, merge, Ci, Co)
+            assert np.array_equal(C.morpho_forward(op, dev(x), dev(w), merge, padding, pv).cpu().numpy(), want), (op, merge, Ci, Co)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("k", [3, 5, 7, 11, (9, 9), (6, 3)])
 def test_morph_kernel_sizes_forward_and_backward(C, k, dtype):
     """Specialised widths (3, 5, 7, 11) and the any-size path, larger channel counts, against the oracle."""
@@ -97,6 +117,30 @@ def test_morph_kernel_sizes_forward_and_backward(C, k, dtype):
                 gx, gw = C.morpho_backward(op, dev(x), dev(w), dev(gy), merge, padding)
                 np.testing.assert_allclose(gx.cpu().numpy(), wgx, **grad_tol(dtype, 10), err_msg=str((op, merge, padding, k)))
                 np.testing.assert_allclose(gw.cpu().numpy(), wgw, **grad_tol(dtype, 100), err_msg=str((op, merge, padding, k)))
+
+
+@pytest.mark.parametrize("k", [(3, 3), (5, 5), (7, 7), (3, 5)])
+@pytest.mark.parametrize("size", [(1, 5, 3), (2, 9, 28), (1, 33, 65), (3, 40, 96)])
+def test_backward_output_channels_divided(C, size, k):
+    """Sum and identity backward where several thread blocks divide the output channels of a tile. Whole-number inputs and gradients: candidates tie, every sum is exact in float, so the
+    gradients are those of the oracle bit for bit whatever the order. With infinities and NaN among the inputs, and a border
+    that leaves pixels without any finite candidate."""
+    rng = np.random.default_rng(size[1] + k[1])
+    B, H, W = size
+    for (Ci, Co) in ((1, 1), (2, 40), (5, 7)):
+        for op, merge, padding in (("dilation", "sum", "replicate"), ("erosion", "sum", "geodesic"), ("erosion", "identity", "zero")):
+            co = Ci if merge == "identity" else Co
+            x = rng.integers(-3, 4, (B, Ci, H, W)).astype(np.float32)
+            bad = rng.random(x.shape)
+            x[bad < 0.2] = -np.inf if op == "dilation" else np.inf
+            x[bad > 0.95] = np.nan
+            x[..., : H // 2 + 1, : W // 2 + 1] = -np.inf if op == "dilation" else np.inf
+            w = rng.integers(-2, 3, (co, 1 if merge == "identity" else Ci, *k)).astype(np.float32)
+            gy = rng.integers(-2, 3, (B, co, H, W)).astype(np.float32)
+            want = O.morpho_backward(op, x, w, gy, merge, padding)
+            got = C.morpho_backward(op, dev(x), dev(w), dev(gy), merge, padding)
+            for name, p, q in zip(("grad_input", "grad_weight"), got, want):
+                assert np.array_equal(p.cpu().numpy(), q), (op, merge, Ci, co, name)
 
 
 def test_saved_indices_equal_recomputed(C):
@@ -348,6 +392,32 @@ def test_smorph_factorised_forward_matches_double(C, case, merge):
     # channels a sum adds up
     scale = ci if merge == "sum" else 1
     torch.testing.assert_close(y.double(), ref, rtol=1e-4, atol=1e-5 * scale * max(1.0, spread))
+
+
+@pytest.mark.parametrize("k", [3, 5, (4, 6)])
+@pytest.mark.parametrize("size", [(1, 7, 8), (2, 28, 28), (1, 70, 97), (1, 224, 224)])
+def test_smorph_forward_channels_divided_in_a_cluster(C, size, k):
+    """Smorph on few tiles: the thread blocks of a cluster divide the input channels, evenly or not, and some hold a single one.
+    Sum, mean, max and the smooth merge against the double kernel, at the bar of the other float smorph tests per channel of a
+    sum, and the double kernel against the oracle; the parts are merged in the order of the ranks, so that a second run gives
+    the same bits."""
+    torch.manual_seed(size[1])
+    B, H, W = size
+    kH, kW = (k, k) if isinstance(k, int) else k
+    for (Ci, Co) in ((1, 3), (5, 4), (9, 6), (20, 13))[: 4 if H < 200 else 2]:
+        x, w = torch.randn(B, Ci, H, W, device="cuda"), 0.3 * torch.randn(Co, Ci, kH, kW, device="cuda")
+        alpha, beta = torch.randn(Co, Ci, device="cuda") * 3, torch.randn(Co, device="cuda")
+        for merge in ("sum", "mean", "max"):
+            got = C.smorph_forward(x, w, alpha, merge)
+            want = C.smorph_forward(x.double(), w.double(), alpha.double(), merge)
+            torch.testing.assert_close(got.double(), want, rtol=1e-4, atol=1e-5 * (Ci if merge == "sum" else 1))
+            assert torch.equal(got, C.smorph_forward(x, w, alpha, merge))
+            if H < 30:
+                reference = O.smorph_forward(x.double().cpu().numpy(), w.double().cpu().numpy(), alpha.double().cpu().numpy(), merge)
+                np.testing.assert_allclose(want.cpu().numpy(), reference, rtol=1e-11, atol=1e-11)
+        got = C.smorph_scm_forward(x, w, alpha, beta)
+        torch.testing.assert_close(got.double(), C.smorph_scm_forward(x.double(), w.double(), alpha.double(), beta.double()), rtol=1e-4, atol=2e-5)
+        assert torch.equal(got, C.smorph_scm_forward(x, w, alpha, beta))
 
 
 @pytest.mark.parametrize("case", [
