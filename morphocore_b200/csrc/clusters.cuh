@@ -35,7 +35,9 @@ template <typename T> __device__ __forceinline__ T load_cluster(uint32_t address
 
 /// CTAs of a cluster that divide the input channels of an item (a tile and a group of output channels) in the smorph forward
 /// kernels: the fewest waves of `per_sm` CTAs per SM, each as long as the channels a CTA walks plus its fixed work (barriers,
-/// first copy, the exchange of the sums) in units of one channel. LEANFIGURES
+/// first copy, the exchange of the sums) in units of one channel. 3 x 3, 32 items of 28 x 28 maps with 8 channels: 20.9 us with
+/// one CTA an item, 14.4 with a cluster; one 224 x 224 image, 64 -> 64 channels (448 items on 296 places): 515 and 465 us;
+/// 5 x 5 on (4, 16, 96, 96) -> 16: 120 and 90 us.
 inline int cluster_size(int64_t items, int channels, int per_sm)
 {
     constexpr int MOST = 8;

@@ -649,9 +649,10 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     const size_t taps = static_cast<size_t>(d.kH) * d.kW;
     const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
     if (items > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
-    // CTAs that divide the output channels of a tile (grid.y); staging its window and adding up grad_input cost one about as
-    // much as four of them.
-    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, 2, 4);
+    // CTAs that divide the output channels of a tile (grid.y). Staging its window and adding up grad_input cost one about as
+    // much as four of them, eight at 3 x 3: there two shares of (16, 32, 56, 56) -> 64 took 317 us, one takes 297; at 5 x 5
+    // two shares of (4, 16, 96, 96) -> 32 take 128 us, one 138.
+    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, 2, sizeof(T) == 4 && KW == 3 ? 8 : 4);
     const dim3 blocks(static_cast<unsigned>(items), static_cast<unsigned>(shares));
     const int channels = a.g.identity ? 1 : (d.Co + shares - 1) / shares;   // the most a CTA walks
     if constexpr (sizeof(T) == 4 && (KW == 3 || KW == 5))

@@ -613,7 +613,8 @@ __global__ void __launch_bounds__(THREADS) morpho_find_tap_kernel(const ForwardA
         int ch = a.idx[at] >> 16;
         ch = min(max(ch, 0), g.Ci - 1);
         const T* xp = a.x + (static_cast<int64_t>(b) * g.Ci + ch) * plane;
-        const T* wk = a.w + static_cast<int64_t>(b) * g.weight_batch_stride + (static_cast<int64_t>(o) * g.Ci + ch) * taps;
+        const T* wk = a.w + static_cast<int64_t>(b) * g.weight_batch_stride + (static_cast<int64_t>(o) * g.Ci + ch) * taps + (g.flipped ? taps - 1 : 0);
+        const int w_step = g.flipped ? -1 : 1;   // wk walks through the structuring element in the order of the taps
         T best = op_init;
         int arg = 0;
         const bool inside = h - (g.kH - 1 - g.pH) >= 0 && h + g.pH < g.H && w - (g.kW - 1 - g.pW) >= 0 && w + g.pW < g.W;
@@ -624,7 +625,8 @@ __global__ void __launch_bounds__(THREADS) morpho_find_tap_kernel(const ForwardA
                 const T* row = xp + static_cast<int64_t>(h + g.pH - kh) * g.W + w + g.pW;
                 for (int kw = 0; kw < g.kW; kw++)
                 {
-                    const T wv = __ldg(wk + g.stored_tap(kh * g.kW + kw));
+                    const T wv = __ldg(wk);
+                    wk += w_step;
                     const T xv = __ldg(row - kw);
                     const T v = IS_MIN ? xv - wv : xv + wv;
                     if (strictly_better<IS_MIN>(v, best))
@@ -641,7 +643,8 @@ __global__ void __launch_bounds__(THREADS) morpho_find_tap_kernel(const ForwardA
                 for (int kw = 0; kw < g.kW; kw++)
                 {
                     const T xv = read_border(xp, g, h + g.pH - kh, w + g.pW - kw, a.fill);
-                    const T wv = __ldg(wk + g.stored_tap(kh * g.kW + kw));
+                    const T wv = __ldg(wk);
+                    wk += w_step;
                     const T v = IS_MIN ? xv - wv : xv + wv;
                     if (strictly_better<IS_MIN>(v, best))
                     {

@@ -768,7 +768,7 @@ struct SmorphForwardArgs
 /// q_i = exp(beta (c_i - ref)), ref = max_i c_i (beta >= 0) or min_i c_i. The channels stream through the CTA, so the
 /// sums are kept relative to the running extremum and rescaled when it moves. The kernel writes the merged value,
 /// or, for the backward pass, ref and 1 / sum_i q_i.
-template <typename T, int KW, int OB, int MODE, bool USE_TMA>
+template <typename T, int KW, int OB, int MODE, bool USE_TMA, bool CLUSTER>
 __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     smorph_forward_kernel(const SmorphForwardArgs<T> a, const __grid_constant__ CUtensorMap tmap)
 {
@@ -793,7 +793,10 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     const bool factorise = FACTOR && a.factorise != 0;
 
     const int tiles = g.tiles_x * g.tiles_y;
-    const int rank = blockIdx.x % a.cluster, item = blockIdx.x / a.cluster;
+    // CLUSTER: the CTAs of a cluster divide the input channels (an instantiation of its own, so that the others keep neither the
+    // bounds of the channels nor the exchange of the parts).
+    const int cluster = CLUSTER ? a.cluster : 1;
+    const int rank = blockIdx.x % cluster, item = blockIdx.x / cluster;
     const int og = item % a.o_groups;
     const int tile = (item / a.o_groups) % tiles;
     const int b = item / (a.o_groups * tiles);
@@ -811,7 +814,7 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     const int wci = g.identity ? 1 : g.Ci;
     const int first_channel = g.identity ? o0 : 0;
     // Input channels of this CTA: all of them, or its part where the CTAs of a cluster divide them.
-    const int c_begin = g.identity ? 0 : share_begin(g.Ci, rank, a.cluster), c_end = g.identity ? 1 : share_begin(g.Ci, rank + 1, a.cluster);
+    const int c_begin = CLUSTER ? share_begin(g.Ci, rank, cluster) : 0, c_end = CLUSTER ? share_begin(g.Ci, rank + 1, cluster) : (g.identity ? 1 : g.Ci);
 
     // Signs of every pair of this CTA: a single sign needs one window per channel, both signs need two.
     bool any_pos = false, any_neg = false;
@@ -1000,6 +1003,7 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
             if (!mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns))
             {
                 if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
+                if constexpr (!CLUSTER) return;
                 failed = true;   // every thread of the CTA waits on the same barrier and gives up together
                 break;           // (the other CTAs of its cluster still wait for it below)
             }
@@ -1116,30 +1120,8 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
 
     const T divisor = static_cast<T>(g.Ci);
     T* dst = STATS ? a.counts : a.y;
-    // One pixel of the result: the merged value, for the smooth merge with the extremum and the sum of its weights.
-    auto store = [&](int o, int rr, int j, T v, T extremum, T sum) {
-        const int h = tile_h0 + ty * PATCH_H + rr, w = tile_w0 + tx * PATCH_W + j;
-        if (o >= o_count || !warp_live || o0 + o_base + o >= g.Co || h >= g.H || w >= g.W) return;
-        const int64_t at = ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w;
-        if constexpr (SOFT)
-        {
-            const T inv = T(1) / sum;
-            if (a.soft_ref != nullptr)
-            {
-                a.soft_ref[at] = extremum;
-                a.soft_inv[at] = inv;
-            }
-            else a.y[at] = v * inv;
-        }
-        else
-        {
-            if (!STATS && a.merge == MC_MERGE_AVERAGE) v = v / divisor;
-            dst[at] = v;
-        }
-    };
-    if (a.cluster == 1)
+    if constexpr (!CLUSTER)
     {
-        if (failed) return;
 #pragma unroll
         for (int o = 0; o < OB; o++)
 #pragma unroll
@@ -1147,78 +1129,117 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
 #pragma unroll
                 for (int j = 0; j < PATCH_W; j++)
                 {
-                    if constexpr (SOFT) store(o, rr, j, merged[o][rr][j], soft_sign[o] * soft_m[o][rr][j], soft_s[o][rr][j]);
-                    else store(o, rr, j, FACTOR ? merged[o][rr][j] + offset[o] : merged[o][rr][j], T(0), T(0));
+                    const int h = tile_h0 + ty * PATCH_H + rr, w = tile_w0 + tx * PATCH_W + j;
+                    if (o >= o_count || !warp_live || o0 + o_base + o >= g.Co || h >= g.H || w >= g.W) continue;
+                    T v = merged[o][rr][j];
+                    const int64_t at = ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w;
+                    if constexpr (SOFT)
+                    {
+                        const T inv = T(1) / soft_s[o][rr][j];
+                        if (a.soft_ref != nullptr)
+                        {
+                            a.soft_ref[at] = soft_sign[o] * soft_m[o][rr][j];
+                            a.soft_inv[at] = inv;
+                        }
+                        else a.y[at] = v * inv;
+                        continue;
+                    }
+                    if constexpr (FACTOR) v += offset[o];
+                    if (!STATS && a.merge == MC_MERGE_AVERAGE) v = v / divisor;
+                    dst[at] = v;
                 }
-        return;
     }
-    // Every CTA of the cluster leaves its part in the place of its windows; rank r merges and stores the pixels r, r + cluster,
-    // ... of every thread, in the order of the ranks.
-    constexpr int PIXELS = OB * PATCH_H * PATCH_W;
-    __syncthreads();   // the windows are no longer read
-    T* slots = sx0 + threadIdx.x;   // [PIXELS][THREADS] merged values; then the offsets [OB], or extrema and sums [PIXELS] each
-#pragma unroll
-    for (int o = 0; o < OB; o++)
+    else
     {
-#pragma unroll
-        for (int p = 0; p < PATCH_H * PATCH_W; p++)
-        {
-            const int at = (o * PATCH_H * PATCH_W + p) * THREADS, rr = p / PATCH_W, j = p % PATCH_W;
-            slots[at] = merged[o][rr][j];
+        // One pixel of the result: the merged value, for the smooth merge with the extremum and the sum of its weights.
+        auto store = [&](int o, int rr, int j, T v, [[maybe_unused]] T extremum, [[maybe_unused]] T sum) {
+            const int h = tile_h0 + ty * PATCH_H + rr, w = tile_w0 + tx * PATCH_W + j;
+            if (o >= o_count || !warp_live || o0 + o_base + o >= g.Co || h >= g.H || w >= g.W) return;
+            const int64_t at = ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w;
             if constexpr (SOFT)
             {
-                slots[PIXELS * THREADS + at] = soft_m[o][rr][j];
-                slots[2 * PIXELS * THREADS + at] = soft_s[o][rr][j];
-            }
-        }
-        if constexpr (!SOFT) slots[(PIXELS + o) * THREADS] = offset[o];
-    }
-    cluster_sync();
-    if (!failed)
-    {
-        const uint32_t mine = smem_addr(slots);
-        auto part = [&](int at, int r) { return load_cluster<T>(mine + at * THREADS * static_cast<int>(sizeof(T)), r); };
-        for (int i = rank; i < PIXELS; i += a.cluster)
-        {
-            const int o = i / (PATCH_H * PATCH_W), rr = i / PATCH_W % PATCH_H, j = i % PATCH_W;
-            T v = part(i, 0);
-            if constexpr (SOFT)
-            {
-                const T bt = o0 + o_base + o < g.Co ? __ldg(a.beta + o0 + o_base + o) : T(0);
-                const T sign = bt >= T(0) ? T(1) : T(-1), scale = exp_scale(bt >= T(0) ? bt : -bt);
-                T top = part(PIXELS + i, 0), sum = part(2 * PIXELS + i, 0);
-                for (int r = 1; r < a.cluster; r++)
+                const T inv = T(1) / sum;
+                if (a.soft_ref != nullptr)
                 {
-                    const T other = part(PIXELS + i, r), higher = top < other ? other : top;
-                    const T keep = soft_exp(top - higher, scale), add = soft_exp(other - higher, scale);
-                    v = fma(v, keep, add * part(i, r));
-                    sum = fma(sum, keep, add * part(2 * PIXELS + i, r));
-                    top = higher;
+                    a.soft_ref[at] = extremum;
+                    a.soft_inv[at] = inv;
                 }
-                store(o, rr, j, v, sign * top, sum);
+                else a.y[at] = v * inv;
             }
             else
             {
-                T off = part(PIXELS + o, 0);
-                for (int r = 1; r < a.cluster; r++)
+                if (!STATS && a.merge == MC_MERGE_AVERAGE) v = v / divisor;
+                dst[at] = v;
+            }
+        };
+        // Every CTA of the cluster leaves its part in the place of its windows; rank r merges and stores the pixels r, r + cluster,
+        // ... of every thread, in the order of the ranks.
+        constexpr int PIXELS = OB * PATCH_H * PATCH_W;
+        __syncthreads();   // the windows are no longer read
+        T* slots = sx0 + threadIdx.x;   // [PIXELS][THREADS] merged values; then the offsets [OB], or extrema and sums [PIXELS] each
+#pragma unroll
+        for (int o = 0; o < OB; o++)
+        {
+#pragma unroll
+            for (int p = 0; p < PATCH_H * PATCH_W; p++)
+            {
+                const int at = (o * PATCH_H * PATCH_W + p) * THREADS, rr = p / PATCH_W, j = p % PATCH_W;
+                slots[at] = merged[o][rr][j];
+                if constexpr (SOFT)
                 {
-                    const T other = part(i, r);
-                    if (!STATS && a.merge == MC_MERGE_MAX) v = v < other ? other : v;
-                    else if (!STATS && a.merge == MC_MERGE_MIN) v = other < v ? other : v;
-                    else v += other;
-                    off += part(PIXELS + o, r);
+                    slots[PIXELS * THREADS + at] = soft_m[o][rr][j];
+                    slots[2 * PIXELS * THREADS + at] = soft_s[o][rr][j];
                 }
-                store(o, rr, j, FACTOR ? v + off : v, T(0), T(0));
+            }
+            if constexpr (!SOFT) slots[(PIXELS + o) * THREADS] = offset[o];
+        }
+        cluster_sync();
+        if (!failed)
+        {
+            const uint32_t mine = smem_addr(slots);
+            auto part = [&](int at, int r) { return load_cluster<T>(mine + at * THREADS * static_cast<int>(sizeof(T)), r); };
+            for (int i = rank; i < PIXELS; i += cluster)
+            {
+                const int o = i / (PATCH_H * PATCH_W), rr = i / PATCH_W % PATCH_H, j = i % PATCH_W;
+                T v = part(i, 0);
+                if constexpr (SOFT)
+                {
+                    const T bt = o0 + o_base + o < g.Co ? __ldg(a.beta + o0 + o_base + o) : T(0);
+                    const T sign = bt >= T(0) ? T(1) : T(-1), scale = exp_scale(bt >= T(0) ? bt : -bt);
+                    T top = part(PIXELS + i, 0), sum = part(2 * PIXELS + i, 0);
+                    for (int r = 1; r < cluster; r++)
+                    {
+                        const T other = part(PIXELS + i, r), higher = top < other ? other : top;
+                        const T keep = soft_exp(top - higher, scale), add = soft_exp(other - higher, scale);
+                        v = fma(v, keep, add * part(i, r));
+                        sum = fma(sum, keep, add * part(2 * PIXELS + i, r));
+                        top = higher;
+                    }
+                    store(o, rr, j, v, sign * top, sum);
+                }
+                else
+                {
+                    T off = part(PIXELS + o, 0);
+                    for (int r = 1; r < cluster; r++)
+                    {
+                        const T other = part(i, r);
+                        if (!STATS && a.merge == MC_MERGE_MAX) v = v < other ? other : v;
+                        else if (!STATS && a.merge == MC_MERGE_MIN) v = other < v ? other : v;
+                        else v += other;
+                        off += part(PIXELS + o, r);
+                    }
+                    store(o, rr, j, FACTOR ? v + off : v, T(0), T(0));
+                }
             }
         }
+        cluster_sync();   // nobody leaves while its part is read
     }
-    cluster_sync();   // nobody leaves while its part is read
 }
 
 template <typename T, int KW, int OB, int MODE, bool USE_TMA>
 int launch_smorph_forward_variant(const SmorphForwardArgs<T>& a, const CUtensorMap& tmap, int64_t blocks, size_t smem, cudaStream_t stream)
 {
-    auto kernel = smorph_forward_kernel<T, KW, OB, MODE, USE_TMA>;
+    auto kernel = a.cluster > 1 ? smorph_forward_kernel<T, KW, OB, MODE, USE_TMA, true> : smorph_forward_kernel<T, KW, OB, MODE, USE_TMA, false>;
     if (a.cluster > 1)   // the parts of a cluster's CTA
         smem = std::max(smem, 128 + static_cast<size_t>(OB) * (MODE == 2 ? 3 * PATCH_H * PATCH_W : PATCH_H * PATCH_W + 1) * THREADS * sizeof(T));
     if (!allow_shared(kernel, smem))
@@ -2149,7 +2170,9 @@ int launch_smorph_backward(const mc_desc& d, const T* x, const T* w, const T* al
     int chunk = static_cast<int>((budget - fixed) / per_o);
     const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
     if (items > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
-    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, (sizeof(T) == 8 || KH >= 5) ? 1 : 2, 2);
+    // The fixed work of a CTA is worth nine channels of the 3 x 3 float kernel (two shares of (4, 16, 96, 96) -> 16: 90 us, one:
+    // 78), and less than two of the others'.
+    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, (sizeof(T) == 8 || KH >= 5) ? 1 : 2, sizeof(T) == 4 && KH == 3 ? 9 : 2);
     chunk = std::max(1, std::min(chunk, a.g.identity ? 1 : (d.Co + shares - 1) / shares));
     a.o_chunk = chunk;
     const size_t smem = fixed + per_o * chunk;

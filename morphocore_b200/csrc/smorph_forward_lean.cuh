@@ -153,7 +153,7 @@ __device__ __forceinline__ void lean_factor_pair(const float4* __restrict__ rows
 template <int KW> constexpr size_t lean_channel_bytes() { return static_cast<size_t>(KW * KW) * LEAN_OB * (sizeof(float2) + sizeof(float)) + LEAN_OB * sizeof(float4); }
 template <int KW> constexpr size_t lean_fixed_bytes() { return 128 + 2 * 128 + 16 + (THREADS / 32) * static_cast<size_t>(LeanTable<KW>::BYTES); }
 
-/// CLUSTER: an instantiation of its own, because the kernel has no register to spare for the bounds of its channels (24.9
+/// CLUSTER: an instantiation of its own, because the kernel has no register to spare for the bounds of its channels (25.4
 /// against 25.6 ms over the two layers of the four-layer model at B = 32).
 template <int KW, bool CLUSTER>
 __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const LeanForwardArgs a, const __grid_constant__ CUtensorMap tmap)
@@ -411,32 +411,56 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
         }
     }
 
-    const float divisor = static_cast<float>(g.Ci);
-    const bool vec_store = (g.W % 4 == 0) && (reinterpret_cast<uintptr_t>(a.y) % 16 == 0);
-    auto store = [&](int o, int rr, float4 v) {
-        const int h = tile_h0 + ty * PATCH_H + rr, w0 = tile_w0 + tx * PATCH_W;
-        if (!warp_live || o >= o_count || o0 + o_base + o >= g.Co || h >= g.H || w0 >= g.W) return;
-        if (a.merge == MC_MERGE_AVERAGE) v = make_float4(v.x / divisor, v.y / divisor, v.z / divisor, v.w / divisor);
-        float* dst = a.y + ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w0;
-        if (vec_store && w0 + PATCH_W <= g.W) *reinterpret_cast<float4*>(dst) = v;
-        else
-        {
-            const float out[PATCH_W] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < PATCH_W; j++)
-                if (w0 + j < g.W) dst[j] = out[j];
-        }
-    };
     if constexpr (!CLUSTER)
     {
+        if (!warp_live) return;
+        const float divisor = static_cast<float>(g.Ci);
+        const bool vec_store = (g.W % 4 == 0) && (reinterpret_cast<uintptr_t>(a.y) % 16 == 0);
 #pragma unroll
         for (int o = 0; o < OB; o++)
+        {
+            if (o >= o_count || o0 + o_base + o >= g.Co) break;
 #pragma unroll
             for (int rr = 0; rr < PATCH_H; rr++)
-                store(o, rr, make_float4(merged[o][rr][0] + offset[o], merged[o][rr][1] + offset[o], merged[o][rr][2] + offset[o], merged[o][rr][3] + offset[o]));
+            {
+                const int h = tile_h0 + ty * PATCH_H + rr, w0 = tile_w0 + tx * PATCH_W;
+                if (h >= g.H || w0 >= g.W) continue;
+                float out[PATCH_W];
+#pragma unroll
+                for (int j = 0; j < PATCH_W; j++)
+                {
+                    const float v = merged[o][rr][j] + offset[o];
+                    out[j] = a.merge == MC_MERGE_AVERAGE ? v / divisor : v;
+                }
+                float* dst = a.y + ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w0;
+                if (vec_store && w0 + PATCH_W <= g.W) *reinterpret_cast<float4*>(dst) = make_float4(out[0], out[1], out[2], out[3]);
+                else
+                {
+#pragma unroll
+                    for (int j = 0; j < PATCH_W; j++)
+                        if (w0 + j < g.W) dst[j] = out[j];
+                }
+            }
+        }
     }
     else
     {
+        const float divisor = static_cast<float>(g.Ci);
+        const bool vec_store = (g.W % 4 == 0) && (reinterpret_cast<uintptr_t>(a.y) % 16 == 0);
+        auto store = [&](int o, int rr, float4 v) {
+            const int h = tile_h0 + ty * PATCH_H + rr, w0 = tile_w0 + tx * PATCH_W;
+            if (!warp_live || o >= o_count || o0 + o_base + o >= g.Co || h >= g.H || w0 >= g.W) return;
+            if (a.merge == MC_MERGE_AVERAGE) v = make_float4(v.x / divisor, v.y / divisor, v.z / divisor, v.w / divisor);
+            float* dst = a.y + ((static_cast<int64_t>(b) * g.Co + o0 + o_base + o) * g.H + h) * g.W + w0;
+            if (vec_store && w0 + PATCH_W <= g.W) *reinterpret_cast<float4*>(dst) = v;
+            else
+            {
+                const float out[PATCH_W] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < PATCH_W; j++)
+                    if (w0 + j < g.W) dst[j] = out[j];
+            }
+        };
         // Every CTA leaves its sums in the place of its windows; rank r adds up and stores rows r, r + cluster, ... of the eight
         // (output channel, patch row) rows of every thread.
         static_assert(OB == 4 && PATCH_W == 4, "a row of the patch and the offsets of the output channels are one float4 each");
