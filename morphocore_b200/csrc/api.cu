@@ -170,6 +170,7 @@ int mc_morpho_backward(const mc_desc* desc, const void* x, const void* w, const 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (empty(desc))
     {
+        if ((desc->flags & MC_FLAG_ACCUMULATE) != 0) return MC_OK;   // nothing to add
         const size_t wn = static_cast<size_t>(desc->Co) * (desc->merge == MC_MERGE_IDENTITY ? 1 : desc->Ci) * desc->kH * desc->kW;
         if (cudaMemsetAsync(gw, 0, wn * (desc->dtype == MC_F32 ? 4 : 8), s) != cudaSuccess) { set_last_error("cudaMemsetAsync failed"); return MC_ERR_CUDA; }
         return MC_OK;

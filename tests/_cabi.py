@@ -7,6 +7,7 @@ import torch
 
 from morphocore_b200 import _native
 
+FLIPPED_WEIGHT, ACCUMULATE = 1, 2   # mc_flags
 MERGES = {"max": 0, "min": 1, "sum": 2, "mean": 3, "smooth": 4, "identity": 5}
 
 
@@ -14,7 +15,7 @@ class Desc(ctypes.Structure):
     _fields_ = [("B", ctypes.c_int32), ("Ci", ctypes.c_int32), ("Co", ctypes.c_int32), ("H", ctypes.c_int32),
                 ("W", ctypes.c_int32), ("kH", ctypes.c_int32), ("kW", ctypes.c_int32), ("op", ctypes.c_int32),
                 ("merge", ctypes.c_int32), ("pad_kind", ctypes.c_int32), ("dtype", ctypes.c_int32),
-                ("reserved", ctypes.c_int32), ("fill", ctypes.c_double), ("weight_batch_stride", ctypes.c_int64)]
+                ("flags", ctypes.c_int32), ("fill", ctypes.c_double), ("weight_batch_stride", ctypes.c_int64)]
 
 
 lib = _native.lib
@@ -33,11 +34,11 @@ def fill_value(op, padding, padding_value, dtype):
     return float("-inf") if op == "dilation" else float("inf")
 
 
-def make_desc(op, x, w, merge, padding="replicate", padding_value=0.0):
+def make_desc(op, x, w, merge, padding="replicate", padding_value=0.0, flags=0):
     B, Ci, H, W = x.shape
     Co, _, kH, kW = w.shape[-4:]
     return Desc(B, Ci, Co, H, W, kH, kW, 0 if op == "dilation" else 1, MERGES[merge], 1 if padding == "replicate" else 0,
-                0 if x.dtype == torch.float32 else 1, 0, fill_value(op, padding, padding_value, x.dtype),
+                0 if x.dtype == torch.float32 else 1, flags, fill_value(op, padding, padding_value, x.dtype),
                 w[0].numel() if w.dim() == 5 else 0)
 
 
@@ -49,8 +50,8 @@ def stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def morpho_forward(op, x, w, merge="sum", padding="replicate", padding_value=0.0, with_index=False):
-    d = make_desc(op, x, w, merge, padding, padding_value)
+def morpho_forward(op, x, w, merge="sum", padding="replicate", padding_value=0.0, with_index=False, flags=0):
+    d = make_desc(op, x, w, merge, padding, padding_value, flags)
     y = torch.empty((d.B, d.Co, d.H, d.W), dtype=x.dtype, device=x.device)
     idx = torch.full(y.shape, -1, dtype=torch.int32, device=x.device) if with_index else None
     check(lib.mc_morpho_forward(ctypes.byref(d), ptr(x), ptr(w), ptr(y), ptr(idx), stream()))
@@ -69,10 +70,10 @@ def morpho_pair_forward(x, w, merge="sum", padding="replicate", padding_value=0.
     return yd, ye
 
 
-def morpho_backward(op, x, w, gy, merge="sum", padding="replicate", padding_value=0.0, idx=None):
-    d = make_desc(op, x, w, merge, padding, padding_value)
-    gx = torch.empty_like(x)
-    gw = torch.empty(w.shape[-4:], dtype=x.dtype, device=x.device)
+def morpho_backward(op, x, w, gy, merge="sum", padding="replicate", padding_value=0.0, idx=None, flags=0, into=None):
+    """Gradients of input and structuring element, in new tensors or in the pair `into`."""
+    d = make_desc(op, x, w, merge, padding, padding_value, flags)
+    gx, gw = into if into is not None else (torch.empty_like(x), torch.empty(w.shape[-4:], dtype=x.dtype, device=x.device))
     need = lib.mc_morpho_backward_workspace_bytes(ctypes.byref(d), 1 if idx is not None else 0)
     ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
     check(lib.mc_morpho_backward(ctypes.byref(d), ptr(x), ptr(w), ptr(idx), ptr(gy), ptr(gx), ptr(gw), ptr(ws), ctypes.c_size_t(need), stream()))

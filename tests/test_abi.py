@@ -43,11 +43,11 @@ class Desc(ctypes.Structure):
     _fields_ = [("B", ctypes.c_int32), ("Ci", ctypes.c_int32), ("Co", ctypes.c_int32), ("H", ctypes.c_int32),
                 ("W", ctypes.c_int32), ("kH", ctypes.c_int32), ("kW", ctypes.c_int32), ("op", ctypes.c_int32),
                 ("merge", ctypes.c_int32), ("pad_kind", ctypes.c_int32), ("dtype", ctypes.c_int32),
-                ("reserved", ctypes.c_int32), ("fill", ctypes.c_double), ("weight_batch_stride", ctypes.c_int64)]
+                ("flags", ctypes.c_int32), ("fill", ctypes.c_double), ("weight_batch_stride", ctypes.c_int64)]
 
 
 def desc(**kw):
-    base = dict(B=1, Ci=2, Co=2, H=8, W=8, kH=3, kW=3, op=0, merge=2, pad_kind=1, dtype=0, reserved=0, fill=0.0, weight_batch_stride=0)
+    base = dict(B=1, Ci=2, Co=2, H=8, W=8, kH=3, kW=3, op=0, merge=2, pad_kind=1, dtype=0, flags=0, fill=0.0, weight_batch_stride=0)
     base.update(kw)
     return Desc(**base)
 
@@ -100,3 +100,13 @@ def test_workspace_sizes(lib):
     # a missing workspace is reported, not dereferenced
     one = ctypes.c_void_p(16)
     assert lib.mc_morpho_backward(ctypes.byref(d), one, one, None, one, one, one, None, ctypes.c_size_t(0), None) == -3
+
+
+def test_accumulate_adds_nothing_for_an_empty_problem(lib):
+    """MC_FLAG_ACCUMULATE: an empty batch or image leaves the weight gradient as it is (no CUDA call is made for it, which is
+    why this runs on host memory)."""
+    gw = (ctypes.c_float * 36)(*range(36))
+    for empty in (dict(B=0), dict(H=0), dict(W=0), dict(B=0, merge=0), dict(B=0, merge=5)):
+        d = desc(flags=2, **empty)
+        assert lib.mc_morpho_backward(ctypes.byref(d), None, None, None, None, None, gw, None, ctypes.c_size_t(0), None) == 0, empty
+        assert list(gw) == list(range(36)), empty

@@ -724,6 +724,26 @@ def test_bounded_wait_runs_out_and_is_counted(C):
     assert C.lib.mc_device_error_count() == 0
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("merge, Ci, Co, k", [("sum", 4, 6, 3), ("mean", 4, 5, 5), ("sum", 4, 5, 7), ("sum", 2, 3, 4), ("max", 4, 5, 3), ("identity", 6, 6, 5),
+                                              ("identity", 6, 6, 11)])
+def test_backward_accumulates_into_what_the_gradients_hold(C, merge, Ci, Co, k, dtype):
+    """MC_FLAG_ACCUMULATE through every backward kernel: two calls into one pair of buffers give the sum of what two plain
+    calls give, and a batch without images in between adds nothing. Gradients are multiples of 1/4 with sums far below
+    2^24, so any order of the atomic additions is exact and the comparison is too."""
+    rng = np.random.default_rng(23)
+    x = [rng.standard_normal((2, Ci, 37, 70)).astype(dtype) for _ in range(2)]
+    gy = [rng.integers(-4, 5, (2, Co, 37, 70)).astype(dtype) for _ in range(2)]
+    w = (0.3 * rng.standard_normal((Co, 1 if merge == "identity" else Ci, k, k))).astype(dtype)
+    for op, flipped in (("dilation", 0), ("erosion", C.FLIPPED_WEIGHT)):
+        plain = [C.morpho_backward(op, dev(a), dev(w), dev(b), merge, flags=flipped) for a, b in zip(x, gy)]
+        into = tuple(torch.full_like(t, 8.0) for t in plain[0])
+        for a, b in ((x[0], gy[0]), (x[0][:0], gy[0][:0]), (x[1], gy[1])):
+            C.morpho_backward(op, dev(a), dev(w), dev(b), merge, flags=flipped | C.ACCUMULATE, into=into)
+        for got, first, second in zip(into, *plain):
+            assert torch.equal(got, 8.0 + first + second), op
+
+
 def test_results_are_reproducible_run_to_run(C):
     """Forward outputs and winner indices are bitwise reproducible; gradients accumulate with atomics and
     agree to rounding."""
