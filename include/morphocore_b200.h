@@ -17,7 +17,8 @@
  *    device share one scratch array. Process state: the per-kernel shared-memory opt-in, the wait limit
  *    (mc_set_wait_limit_ns), the launch counter and, per device, the counter of timed-out waits
  *    (mc_device_error_count), which hosts should poll at their own synchronisation points: a thread block whose
- *    wait ran out returns without writing its tile, and the call that launched it has long returned MC_OK.
+ *    wait ran out returns without writing its tile (where the blocks of a cluster share a tile, none of them writes
+ *    it), and the call that launched it has long returned MC_OK.
  */
 #ifndef MORPHOCORE_B200_H
 #define MORPHOCORE_B200_H
@@ -179,9 +180,10 @@ int mc_device_error_reset(void);
  * from now on (default 1 s). No counterpart in the reference. */
 int mc_set_wait_limit_ns(uint64_t limit_ns);
 
-/* Self-test of the time-out path: queues one thread block that waits, with the same bounded wait as the kernels,
- * for a copy that is never issued. After limit_ns (at most 1 s) it gives up, adds one to the counter of
- * mc_device_error_count and returns; the context stays usable. No counterpart in the reference. */
+/* Self-test of the time-out path: queues a cluster of two thread blocks, one of which waits, with the same bounded wait as
+ * the kernels, for a copy that is never issued. After limit_ns (at most 1 s) it gives up and adds one to the counter of
+ * mc_device_error_count, the other block learns of it, and both return; the context stays usable. No counterpart in the
+ * reference. */
 int mc_selftest_wait_timeout(uint64_t limit_ns, void* stream);
 
 /* Number of kernels this library has launched in the calling process since it was loaded. */

@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstdio>
 
+#include "clusters.cuh"
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -32,25 +33,36 @@ static std::atomic<uint64_t> g_wait_limit_ns{1000000000ull};  // one second
 
 uint64_t wait_limit_ns() { return g_wait_limit_ns.load(std::memory_order_relaxed); }
 
-/// One CTA that waits, with the bounded wait of the TMA kernels, on an mbarrier that expects 16 bytes which no copy
-/// ever delivers: the wait runs out after limit_ns, the CTA counts the time-out and returns. Nothing faults or
-/// spins; this is how the time-out path is exercised.
+/// A cluster of two CTAs that waits, with the bounded wait of the TMA kernels, for copies that nobody ever issues: the wait of
+/// CTA 0 expects 16 bytes and runs out after limit_ns for every second thread, while the others take their copy as landed
+/// (threads time their waits one by one, a copy may land just then); CTA 1 has nothing to wait for. CTA 0 must leave as one and
+/// count its time-out, and CTA 1 must learn of it at the barrier of the exchange; a protocol that fails in either counts once
+/// more. Nothing faults or spins; this is how the time-out path is exercised.
 __global__ void wait_timeout_selftest_kernel(unsigned int* errors, uint64_t limit_ns)
 {
-    __shared__ uint64_t bar;
+    __shared__ uint64_t full[2];
+    __shared__ uint32_t gave_up;
+    const int rank = blockIdx.x;
     if (threadIdx.x == 0)
     {
-        mbar_init(&bar, 1);
+        mbar_init(full, 1);
+        mbar_init(full + 1, 1);
         mbar_fence_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0) mbar_expect_tx(&bar, 16);
+    if (threadIdx.x == 0 && rank == 0) mbar_expect_tx(full, 16);
     __syncthreads();
-    if (!mbar_wait(&bar, 0, limit_ns))
+    bool landed = true;
+    if (rank == 0 && threadIdx.x % 2 == 0) landed = mbar_wait(full, 0, limit_ns);
+    if (cta_gave_up(landed))
     {
-        if (threadIdx.x == 0 && errors != nullptr) atomicAdd(errors, 1u);
+        if (rank != 0 && threadIdx.x == 0 && errors != nullptr) atomicAdd(errors, 1u);   // CTA 1 had nothing to wait for
+        leave_cluster(&gave_up, full, 0, 0, errors, limit_ns);                           // no copy was issued
         return;
     }
+    const bool complete = cluster_complete(&gave_up, 2);
+    if (threadIdx.x == 0 && errors != nullptr && (rank == 0 || complete)) atomicAdd(errors, 1u);
+    cluster_sync();
 }
 
 static thread_local char g_last_error[512] = "";
@@ -386,8 +398,8 @@ int mc_selftest_wait_timeout(uint64_t limit_ns, void* stream)
         set_last_error("mc_selftest_wait_timeout: limit of 1 ns .. 1 s expected");
         return MC_ERR_INVALID_ARGUMENT;
     }
-    wait_timeout_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(device_error_counter(), limit_ns);
-    return check_launch("wait_timeout_selftest_kernel");
+    return launch_clusters(wait_timeout_selftest_kernel, 2, 1, 0, static_cast<cudaStream_t>(stream), "wait_timeout_selftest_kernel",
+                           device_error_counter(), limit_ns);
 }
 
 uint64_t mc_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }

@@ -4,6 +4,7 @@
 
 #include "common.cuh"
 #include "shares.cuh"
+#include "tma.cuh"
 
 namespace mc
 {
@@ -11,6 +12,7 @@ namespace mc
 /// Barrier over the thread blocks of a cluster: what they wrote to shared memory before it is visible to the others after it.
 __device__ __forceinline__ void cluster_sync()
 {
+    __syncwarp();   // .aligned: the warp arrives as one
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 /// Reads of the shared memory of the cluster's block `rank`, at the place that `address` has in the reader's own.
@@ -31,6 +33,40 @@ template <typename T> __device__ __forceinline__ T load_cluster(uint32_t address
         asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f64 %0, [a];\n\t}"
                      : "=d"(v) : "r"(address), "r"(rank) : "memory");
     return v;
+}
+
+// A wait on a copy that runs out must not keep the other CTAs of the cluster at its barriers. Threads time their waits one by
+// one, and where the copy lands just then some of them give up and others do not: so the CTA decides as one (cta_gave_up), in
+// place of the barrier that follows the wait, and then leaves the kernel as one (leave_cluster), through the same two cluster
+// barriers as its peers, which learn of it at the first (cluster_complete) and store nothing.
+
+__device__ __forceinline__ bool cta_gave_up(bool landed) { return __syncthreads_or(!landed) != 0; }
+
+/// The barrier between writing the parts and merging them; true where every CTA of the cluster has written its own. `gave_up`:
+/// a word of shared memory. A second cluster_sync follows when the parts have been read.
+__device__ __forceinline__ bool cluster_complete(uint32_t* gave_up, int cluster)
+{
+    if (threadIdx.x == 0) *gave_up = 0;
+    cluster_sync();
+    const int rank = threadIdx.x & 31;
+    uint32_t flag = 0;
+    if (rank < cluster)
+        asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u32 %0, [a];\n\t}"
+                     : "=r"(flag) : "r"(smem_addr(gave_up)), "r"(rank) : "memory");
+    return !__any_sync(0xffffffffu, flag != 0);
+}
+
+/// What a CTA that gave up does instead of writing and merging parts; it returns afterwards. Thread 0 counts it and waits, once
+/// more with a limit, for the `copies` copies still in flight (on barriers with copy n's on full[n & 1], from copy `first` on),
+/// so that the shared memory they write is not given back before they have landed.
+__device__ __forceinline__ void leave_cluster(uint32_t* gave_up, uint64_t* full, int first, int copies, unsigned int* errors, uint64_t limit_ns)
+{
+    if (threadIdx.x == 0) *gave_up = 1;
+    cluster_sync();
+    cluster_sync();
+    if (threadIdx.x != 0) return;
+    if (errors != nullptr) atomicAdd(errors, 1u);
+    for (int n = first; n < first + copies; n++) mbar_wait(full + (n & 1), (n >> 1) & 1, limit_ns > 1000000000ull ? limit_ns : 1000000000ull);
 }
 
 /// CTAs of a cluster that divide the input channels of an item (a tile and a group of output channels) in the smorph forward

@@ -777,9 +777,10 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
     const Geometry& g = a.g;
     const int taps = g.taps();
     const int welems = g.window_elems();
-    // Layout: [2 mbarriers][pad to 128][stage 0][stage 1 (TMA only)][weights][signs and scales]; a stage is
+    // Layout: [2 mbarriers][flag of a cluster's CTA][pad to 128][stage 0][stage 1 (TMA only)][weights][signs and scales]; a stage is
     // [slot][chunk][window]: slot 0 read by pairs of the CTA's first sign, slot 1 by the other sign if any.
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);
+    [[maybe_unused]] uint32_t* gave_up = reinterpret_cast<uint32_t*>(full + 2);
     const int slot_elems = (a.chunk * welems * static_cast<int>(sizeof(T)) + 127) / 128 * 128 / static_cast<int>(sizeof(T));
     T* sx0 = reinterpret_cast<T*>(smem_raw + 128);
     T* sw = sx0 + (USE_TMA ? 2 : 1) * 2 * slot_elems;   // [2 chunk][taps][OB], sign folded
@@ -915,7 +916,6 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
         return stage + (c >= a.chunk ? slot_elems + (c - a.chunk) * welems : c * welems);
     };
     int n = 0;
-    bool failed = false;
     for (int c0 = c_begin; c0 < c_end; c0 += span, n++)
     {
         const int cc = min(span, c_end - c0);
@@ -998,24 +998,32 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
                 }
             }
         }
+        [[maybe_unused]] bool landed = true;
         if constexpr (USE_TMA)
         {
-            if (!mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns))
+            landed = mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns);
+            if constexpr (!CLUSTER)
+                if (!landed)
+                {
+                    if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
+                    return;
+                }
+            if (border)   // harmless where the copy has not landed
             {
-                if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
-                if constexpr (!CLUSTER) return;
-                failed = true;   // every thread of the CTA waits on the same barrier and gives up together
-                break;           // (the other CTAs of its cluster still wait for it below)
-            }
-            if (border)
-            {
-                const T* src = xb + static_cast<int64_t>(first_channel + c0) * plane;
                 fix_window_border(stage, min(cc, a.chunk), g, tile_h0, tile_w0, fill0);
                 if (mixed) fix_window_border(stage + slot_elems, cc, g, tile_h0, tile_w0, Limits<T>::big());
                 else if (cc > a.chunk) fix_window_border(stage + slot_elems, cc - a.chunk, g, tile_h0, tile_w0, fill0);
             }
         }
-        __syncthreads();
+        if constexpr (USE_TMA && CLUSTER)
+        {
+            if (cta_gave_up(landed))
+            {
+                leave_cluster(gave_up, full, n, 1 + (c0 + span < c_end), a.errors, a.wait_limit_ns);
+                return;
+            }
+        }
+        else __syncthreads();
 
         for (int c = 0; c < cc && warp_live; c++)
         {
@@ -1193,8 +1201,7 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 1 : 2)
             }
             if constexpr (!SOFT) slots[(PIXELS + o) * THREADS] = offset[o];
         }
-        cluster_sync();
-        if (!failed)
+        if (cluster_complete(gave_up, cluster))
         {
             const uint32_t mine = smem_addr(slots);
             auto part = [&](int at, int r) { return load_cluster<T>(mine + at * THREADS * static_cast<int>(sizeof(T)), r); };

@@ -167,6 +167,7 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
     const Geometry& g = a.g;
 
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);
+    [[maybe_unused]] uint32_t* gave_up = reinterpret_cast<uint32_t*>(full + 2);
     const int stage_elems = (a.chunk * WELEMS * 4 + 127) / 128 * 128 / 4;
     float* sx0 = reinterpret_cast<float*>(smem_raw + 128);                      // two stages of `chunk` raw windows
     float4* spar = reinterpret_cast<float4*>(sx0 + 2 * stage_elems);            // [chunk][OB]: sign, exp scale, Mw, range of s w
@@ -247,7 +248,6 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
     }
 
     int n = 0;
-    bool failed = false;
     for (int c0 = c_begin; c0 < c_end; c0 += a.chunk, n++)
     {
         const int cc = min(a.chunk, c_end - c0);
@@ -293,14 +293,24 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
                 sw[(c * TAPS + k) * OB + o] = v;
             }
         }
-        if (!mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns))
+        const bool landed = mbar_wait(full + (n & 1), (n >> 1) & 1, a.wait_limit_ns);
+        if constexpr (CLUSTER)
         {
-            if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
-            if constexpr (!CLUSTER) return;
-            failed = true;   // every thread of the CTA waits on the same barrier and gives up together
-            break;           // (the other CTAs of its cluster still wait for it below)
+            if (cta_gave_up(landed))
+            {
+                leave_cluster(gave_up, full, n, 1 + (c0 + a.chunk < c_end), a.errors, a.wait_limit_ns);
+                return;
+            }
         }
-        __syncthreads();
+        else
+        {
+            if (!landed)
+            {
+                if (threadIdx.x == 0 && a.errors != nullptr) atomicAdd(a.errors, 1u);
+                return;
+            }
+            __syncthreads();
+        }
         if (!warp_live) continue;
 
         for (int c = 0; c < cc; c++)
@@ -472,8 +482,7 @@ __global__ void __launch_bounds__(THREADS, 2) smorph_forward_lean_kernel(const L
             for (int rr = 0; rr < PATCH_H; rr++)
                 slots[(o * PATCH_H + rr) * THREADS] = make_float4(merged[o][rr][0], merged[o][rr][1], merged[o][rr][2], merged[o][rr][3]);
         slots[OB * PATCH_H * THREADS] = make_float4(offset[0], offset[1], offset[2], offset[3]);
-        cluster_sync();
-        if (!failed)
+        if (cluster_complete(gave_up, cluster))
         {
             const uint32_t mine = smem_addr(slots);
             for (int i = rank; i < OB * PATCH_H; i += cluster)

@@ -705,8 +705,10 @@ def test_tma_staged_shapes_all_paddings(C, dtype):
 
 
 def test_bounded_wait_runs_out_and_is_counted(C):
-    """The time-out path of the TMA kernels without a fault: one thread block waits 2 ms for a copy that nobody
-    issues, gives up, counts itself and returns. The context stays usable (a forward pass runs right after) and the
+    """The time-out path of the TMA kernels without a fault: one of the two thread blocks of a cluster waits 2 ms for a
+    copy that nobody issues. Half of its threads see the wait run out, the others take their copy as landed (a copy may land
+    at that very moment): the block leaves as one and counts itself once, and its peer learns of it at the cluster's barrier
+    (the kernel counts once more if it does not). The context stays usable (a forward pass runs right after) and the
     counter reads one more than before; it is then set back so that the session ends at zero."""
     import time
     before = C.lib.mc_device_error_count()
