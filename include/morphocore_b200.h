@@ -43,11 +43,12 @@ enum mc_merge { MC_MERGE_MAX = 0, MC_MERGE_MIN = 1, MC_MERGE_ADD = 2, MC_MERGE_A
  * CPP/morpho_padding_policy.hpp:23-33) or the clamped edge pixel. */
 enum mc_pad_kind { MC_PAD_FILL = 0, MC_PAD_REPLICATE = 1 };
 
-/* Bits of mc_desc.flags, dilation / erosion functions only.
+/* Bits of mc_desc.flags, dilation / erosion functions only: the smorph functions, and any other bit, are refused with
+ * MC_ERR_INVALID_ARGUMENT.
  * FLIPPED_WEIGHT: w is read, and gw written, with both kernel axes reversed: the operation works with w[kH-1-kh, kW-1-kw]
  *   at tap (kh, kw). It is how the Python layer's erosion hands over the structuring element as the user holds it
  *   (the reference flips a copy first, morphocore/functional/erosion.py:89).
- * ACCUMULATE: the backward functions add to what gx and gw hold instead of overwriting them. */
+ * ACCUMULATE: the backward functions add to what gx and gw hold instead of overwriting them (the forward functions ignore it). */
 enum mc_flags { MC_FLAG_FLIPPED_WEIGHT = 1, MC_FLAG_ACCUMULATE = 2 };
 
 enum mc_dtype { MC_F32 = 0, MC_F64 = 1 };
@@ -55,7 +56,7 @@ enum mc_dtype { MC_F32 = 0, MC_F64 = 1 };
 enum mc_status
 {
     MC_OK = 0,
-    MC_ERR_INVALID_ARGUMENT = -1, /* NULL pointer, non-positive size, unknown enum, identity with Co != Ci */
+    MC_ERR_INVALID_ARGUMENT = -1, /* NULL pointer, non-positive size, unknown enum or flag, identity with Co != Ci */
     MC_ERR_UNSUPPORTED = -2,      /* structuring element too large for shared memory or for packed indices */
     MC_ERR_WORKSPACE = -3,        /* workspace smaller than mc_*_workspace_bytes() */
     MC_ERR_CUDA = -4              /* a CUDA runtime call failed; mc_last_error() has the message */

@@ -107,6 +107,11 @@ int validate(const mc_desc* d, bool morph, bool smooth)
         set_last_error("the smooth channel merge exists for smorph only and has its own entry points, mc_smorph_scm_*");
         return MC_ERR_UNSUPPORTED;
     }
+    if ((d->flags & ~(morph ? MC_FLAG_FLIPPED_WEIGHT | MC_FLAG_ACCUMULATE : 0)) != 0)
+    {
+        set_last_error(morph ? "unknown bits in flags (0x%x)" : "the smorph functions take no flags (0x%x)", static_cast<unsigned>(d->flags));
+        return MC_ERR_INVALID_ARGUMENT;
+    }
     if (d->merge == MC_MERGE_IDENTITY && d->Co != d->Ci)
     {
         set_last_error("Identity mode requires weight.shape[0] == input.shape[1]");

@@ -105,6 +105,24 @@ def smorph_backward(x, w, alpha, y, gy, merge="sum"):
     return gx, gw, ga
 
 
+def smorph_reparametrise(w, alpha, merge="sum"):
+    """The re-parametrised structuring element of [Co, Ci, kH, kW] weights and one alpha per pair."""
+    Ci = w.shape[0] if merge == "identity" else w.shape[1]
+    d = make_desc("dilation", torch.empty((1, Ci, 1, 1), dtype=w.dtype), w, merge)
+    out = torch.empty_like(w)
+    check(lib.mc_smorph_reparametrise(ctypes.byref(d), ptr(w), ptr(alpha), ptr(out), stream()))
+    return out
+
+
+def smorph_reparametrise_backward(w, alpha, g, galpha, merge="sum"):
+    """Gradient of w; adds to `galpha` what flows through the re-parametrised structuring element."""
+    Ci = w.shape[0] if merge == "identity" else w.shape[1]
+    d = make_desc("dilation", torch.empty((1, Ci, 1, 1), dtype=w.dtype), w, merge)
+    gw = torch.empty_like(w)
+    check(lib.mc_smorph_reparametrise_backward(ctypes.byref(d), ptr(w), ptr(alpha), ptr(g), ptr(gw), ptr(galpha), stream()))
+    return gw
+
+
 def smorph_scm_forward(x, w, alpha, beta):
     d = make_desc("dilation", x, w, "smooth")
     a = pair_alphas(alpha, d.Co, d.Ci, "sum")

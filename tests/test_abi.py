@@ -110,3 +110,27 @@ def test_accumulate_adds_nothing_for_an_empty_problem(lib):
         d = desc(flags=2, **empty)
         assert lib.mc_morpho_backward(ctypes.byref(d), None, None, None, None, None, gw, None, ctypes.c_size_t(0), None) == 0, empty
         assert list(gw) == list(range(36)), empty
+
+
+def test_flags_are_checked(lib):
+    """Unknown bits are refused everywhere, every bit by the smorph functions; the known ones pass where they mean something."""
+    one, no = ctypes.c_void_p(16), ctypes.c_size_t(0)   # never dereferenced
+    hard = {"mc_morpho_forward": (one, one, one, None, None), "mc_morpho_pair_forward": (one, one, one, one, None),
+            "mc_morpho_backward": (one, one, None, one, one, one, None, no, None), "mc_morpho_backward_noalloc": (one, one, one, one, one, None)}
+    smooth = {"mc_smorph_forward": (one, one, one, one, None), "mc_smorph_backward": (one,) * 8 + (None, no, None),
+              "mc_smorph_reparametrise": (one, one, one, None), "mc_smorph_reparametrise_backward": (one, one, one, one, one, None)}
+    scm = {"mc_smorph_scm_forward": (one,) * 5 + (None,), "mc_smorph_scm_backward": (one,) * 10 + (None, no, None)}
+    for name, args in hard.items():
+        for flags in (4, 8 | 1, -1, 1 << 30):
+            assert getattr(lib, name)(ctypes.byref(desc(B=0, flags=flags)), *args) == -1, (name, flags)
+            assert b"unknown bits" in lib.mc_last_error()
+    for flags in (1, 2, 3):   # an empty batch is a valid no-op (the backward functions clear the weight gradient unless they accumulate)
+        for name, args in hard.items():
+            if "backward" not in name or flags & 2:
+                assert getattr(lib, name)(ctypes.byref(desc(B=0, flags=flags)), *args) == 0, (name, flags)
+    for names, merge in ((smooth, 2), (scm, 4)):
+        for name, args in names.items():
+            for flags in (1, 2, 3, 4):
+                assert getattr(lib, name)(ctypes.byref(desc(B=0, merge=merge, flags=flags)), *args) == -1, (name, flags)
+                assert b"no flags" in lib.mc_last_error()
+    assert lib.mc_smorph_forward(ctypes.byref(desc(B=0)), *smooth["mc_smorph_forward"]) == 0

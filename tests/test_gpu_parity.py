@@ -746,6 +746,54 @@ def test_backward_accumulates_into_what_the_gradients_hold(C, merge, Ci, Co, k, 
             assert torch.equal(got, 8.0 + first + second), op
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("merge, Ci, Co, k", [("sum", 4, 6, 3), ("mean", 4, 5, 5), ("sum", 4, 5, 7), ("sum", 2, 3, 4), ("max", 4, 5, 3), ("identity", 6, 6, 5),
+                                              ("identity", 6, 6, 11)])
+def test_flipped_weight_is_the_flipped_structuring_element(C, merge, Ci, Co, k, dtype):
+    """MC_FLAG_FLIPPED_WEIGHT: the result, the winner index and the gradients of a call that is handed the flipped copy, the
+    weight gradient flipped back. Gradients as above: exact in any order."""
+    rng = np.random.default_rng(24)
+    x = rng.standard_normal((2, Ci, 37, 70)).astype(dtype)
+    gy = rng.integers(-4, 5, (2, Co, 37, 70)).astype(dtype)
+    w = dev((0.3 * rng.standard_normal((Co, 1 if merge == "identity" else Ci, k, k))).astype(dtype))
+    for op in ("dilation", "erosion"):
+        wf = w.flip((-2, -1)).contiguous()
+        want, want_idx = C.morpho_forward(op, dev(x), wf, merge, with_index=True)
+        got, got_idx = C.morpho_forward(op, dev(x), w, merge, with_index=True, flags=C.FLIPPED_WEIGHT)
+        assert torch.equal(got, want) and torch.equal(got_idx, want_idx), op
+        idx = want_idx if merge == "max" else None
+        wgx, wgw = C.morpho_backward(op, dev(x), wf, dev(gy), merge, idx=idx)
+        for kept in {idx is not None, False}:
+            gx, gw = C.morpho_backward(op, dev(x), w, dev(gy), merge, idx=idx if kept else None, flags=C.FLIPPED_WEIGHT)
+            assert torch.equal(gx, wgx) and torch.equal(gw, wgw.flip((-2, -1))), (op, kept)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("merge, Co, Ci, kH, kW", [("sum", 5, 3, 3, 3), ("sum", 2, 7, 5, 7), ("identity", 6, 1, 3, 3), ("smooth", 3, 4, 1, 2), ("sum", 9, 40, 11, 11)])
+def test_reparametrisation_and_its_gradient(C, merge, Co, Ci, kH, kW, dtype):
+    """mc_smorph_reparametrise and its backward against the formulas in double: t (1 -+ t) / 2, each weight is the sum of two
+    products (four roundings, 2^-22 of the terms' size in float), the alpha gradient a sum of kH kW products that is ADDED to
+    what the buffer holds."""
+    rng = np.random.default_rng(25)
+    w, g = rng.standard_normal((2, Co, Ci, kH, kW)).astype(dtype)
+    alpha, held = rng.standard_normal((2, Co, Ci)).astype(dtype)
+    eps = float(np.finfo(dtype).eps)
+    wd, gd, t = w.astype(np.float64), g.astype(np.float64), np.tanh(alpha.astype(np.float64))[..., None, None]
+    flip = lambda a: a[..., ::-1, ::-1]
+    s = (1 - t) / 2 * flip(wd) + (1 + t) / 2 * wd
+    scale = np.maximum(np.abs(wd), flip(np.abs(wd)))
+    got = C.smorph_reparametrise(dev(w), dev(alpha), merge).cpu().numpy()
+    assert (np.abs(got - t * s) <= 8 * eps * scale + 1e-300).all()
+    galpha = dev(held)
+    gw = C.smorph_reparametrise_backward(dev(w), dev(alpha), dev(g), galpha, merge).cpu().numpy()
+    assert (np.abs(gw - (t * (1 + t) / 2 * gd + t * (1 - t) / 2 * flip(gd))) <= 8 * eps * np.maximum(np.abs(gd), flip(np.abs(gd)))).all()
+    terms = gd * (s + t * (wd - flip(wd)) / 2)
+    want = held + ((1 - t * t) * terms).sum((-2, -1))
+    # |wd| + |flip(wd)| bounds both parts of a term; kH kW additions and the cancellation in 1 - t^2 on top
+    bound = (np.abs(gd) * (np.abs(wd) + flip(np.abs(wd)))).sum((-2, -1)) * (kH * kW / 32 + 16) * eps + np.abs(want) * 4 * eps
+    assert (np.abs(galpha.cpu().numpy() - want) <= bound).all()
+
+
 def test_results_are_reproducible_run_to_run(C):
     """Forward outputs and winner indices are bitwise reproducible; gradients accumulate with atomics and
     agree to rounding."""
