@@ -234,7 +234,10 @@ struct PairsBackwardArgs
 /// tracked strict comparison (kh-major, kw order: the first tap wins ties, index 0 when nothing beats the
 /// initial value). Gradients are accumulated in a shared window (grad_input, halo dropped at the flush)
 /// and in interleaved shared bins (grad_weight), then flushed with global atomics.
-template <typename T, bool IS_MIN, int KW, int OB>
+/// SHARED: several CTAs (grid.y) may divide the output channels of a tile, see channel_shares. The any-size float kernel for four
+/// channels has an instantiation of its own without, because it has no register to spare for the bounds: (4, 16, 96, 96) -> 20,
+/// 570 against 602 us at 9 x 9, 524 against 614 at 8 x 8, 948 against 1022 at 13 x 13.
+template <typename T, bool IS_MIN, int KW, int OB, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_kernel(const PairsBackwardArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -265,8 +268,8 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_kernel(const
     for (int e = threadIdx.x; e < g.window_elems(); e += THREADS) sg[e] = T(0);
     for (int e = threadIdx.x; e < OB * taps * a.copies; e += THREADS) bins[e] = T(0);
 
-    const int o_begin = g.identity ? ci : share_begin(g.Co, blockIdx.y, gridDim.y);
-    const int o_end = g.identity ? ci + 1 : share_begin(g.Co, blockIdx.y + 1, gridDim.y);
+    const int o_begin = g.identity ? ci : (SHARED ? share_begin(g.Co, blockIdx.y, gridDim.y) : 0);
+    const int o_end = g.identity ? ci + 1 : (SHARED ? share_begin(g.Co, blockIdx.y + 1, gridDim.y) : g.Co);
     for (int o0 = o_begin; o0 < o_end; o0 += OB)
     {
         __syncthreads();
@@ -707,7 +710,9 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     a.copies = bin_copies(taps * OB, sizeof(T), std::min<size_t>(32 * 1024, MAX_SHARED_BYTES - fixed));
     if (a.copies < 1) a.copies = 1;
     const size_t smem = fixed + taps * OB * a.copies * sizeof(T);
-    auto kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB>;
+    auto kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB, true>;
+    if constexpr (KW == 0 && sizeof(T) == 4 && OB > 1)
+        if (shares == 1) kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB, false>;
     if (!allow_shared(kernel, smem)) { set_last_error("cannot opt in to %zu bytes of shared memory", smem); return MC_ERR_UNSUPPORTED; }
     kernel<<<blocks, THREADS, smem, stream>>>(a);
     return check_launch("morpho_backward_pairs_kernel");
