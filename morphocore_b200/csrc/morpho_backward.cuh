@@ -652,34 +652,40 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     const size_t taps = static_cast<size_t>(d.kH) * d.kW;
     const int64_t items = static_cast<int64_t>(a.g.tiles_x) * a.g.tiles_y * d.Ci * d.B;
     if (items > 0x7fffffffLL) { set_last_error("too many tiles for one launch"); return MC_ERR_UNSUPPORTED; }
-    // CTAs that divide the output channels of a tile (grid.y). Staging its window and adding up grad_input cost one about as
-    // much as four of them, eight at 3 x 3: there two shares of (16, 32, 56, 56) -> 64 took 317 us, one takes 297; at 5 x 5
-    // two shares of (4, 16, 96, 96) -> 32 take 128 us, one 138.
-    const int shares = a.g.identity ? 1 : channel_shares(items, d.Co, 2, sizeof(T) == 4 && KW == 3 ? 8 : 4);
-    const dim3 blocks(static_cast<unsigned>(items), static_cast<unsigned>(shares));
-    const int channels = a.g.identity ? 1 : (d.Co + shares - 1) / shares;   // the most a CTA walks
+    // CTAs that divide the output channels of a tile (grid.y), for a kernel that computes `group` of them together. Staging its
+    // window and adding up grad_input cost one about as much as two of them where four are computed together, three in double;
+    // channel by channel eight at 3 x 3 (two shares of (16, 32, 56, 56) -> 64 took 317 us, one takes 297) and five at 5 x 5 (two
+    // of (4, 16, 96, 96) -> 32 take 128 us, one 138; two of 104 tiles with four channels 18.8, one 17.6).
+    auto shares_of = [&](int group) {
+        if (a.g.identity) return 1;
+        return group == 4 ? channel_shares(items, d.Co, 2, 2, 4, 0.7) : channel_shares(items, d.Co, 2, sizeof(T) == 8 ? 3 : (KW == 3 ? 8 : 5), group);
+    };
+    auto most_channels = [&](int shares) { return a.g.identity ? 1 : (d.Co + shares - 1) / shares; };   // that one CTA walks
+    auto grid = [&](int shares) { return dim3(static_cast<unsigned>(items), static_cast<unsigned>(shares)); };
     if constexpr (sizeof(T) == 4 && (KW == 3 || KW == 5))
     {
-        const size_t bytes = pairs_regs_smem<KW>(a.g, channels);
+        const int shares = shares_of(1);
+        const size_t bytes = pairs_regs_smem<KW>(a.g, most_channels(shares));
         if (bytes > 0)
         {
             auto fast = morpho_backward_pairs_regs_kernel<IS_MIN, KW>;
             if (allow_shared(fast, bytes))
             {
-                fast<<<blocks, THREADS, bytes, stream>>>(a);
+                fast<<<grid(shares), THREADS, bytes, stream>>>(a);
                 return check_launch("morpho_backward_pairs_regs_kernel");
             }
         }
     }
     if constexpr (sizeof(T) == 4 && (KW == 3 || KW == 5 || KW == 7))
     {
-        const size_t bytes = pairs_rows_smem<KW>(a.g, channels);
+        const int shares = shares_of(ROWS_GROUP);
+        const size_t bytes = pairs_rows_smem<KW>(a.g, most_channels(shares));
         if (bytes > 0)
         {
             auto fast = morpho_backward_pairs_rows_kernel<IS_MIN, KW>;
             if (allow_shared(fast, bytes))
             {
-                fast<<<blocks, THREADS, bytes, stream>>>(a);
+                fast<<<grid(shares), THREADS, bytes, stream>>>(a);
                 return check_launch("morpho_backward_pairs_rows_kernel");
             }
         }
@@ -710,11 +716,12 @@ int launch_backward_pairs(const mc_desc& d, const T* x, const T* w, const T* gy,
     a.copies = bin_copies(taps * OB, sizeof(T), std::min<size_t>(32 * 1024, MAX_SHARED_BYTES - fixed));
     if (a.copies < 1) a.copies = 1;
     const size_t smem = fixed + taps * OB * a.copies * sizeof(T);
+    const int shares = shares_of(OB);
     auto kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB, true>;
     if constexpr (KW == 0 && sizeof(T) == 4 && OB > 1)
         if (shares == 1) kernel = morpho_backward_pairs_kernel<T, IS_MIN, KW, OB, false>;
     if (!allow_shared(kernel, smem)) { set_last_error("cannot opt in to %zu bytes of shared memory", smem); return MC_ERR_UNSUPPORTED; }
-    kernel<<<blocks, THREADS, smem, stream>>>(a);
+    kernel<<<grid(shares), THREADS, smem, stream>>>(a);
     return check_launch("morpho_backward_pairs_kernel");
 }
 

@@ -6,6 +6,8 @@
 namespace mc
 {
 
+constexpr int ROWS_GROUP = 4;   // output channels the kernel computes together
+
 ///  - Tap search: a first pass takes the extremum of every kernel row with the 3-input max and keeps the
 ///    FIRST row that strictly improves on the running best (rows ascend, so ties go to the lower kh); a
 ///    second pass scans that one row, from the last column down, for the lowest kw whose value equals the
@@ -22,7 +24,7 @@ template <bool IS_MIN, int KW>
 __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_rows_kernel(const PairsBackwardArgs<float> a)
 {
     using T = float;
-    constexpr int OB = 4, WARPS = THREADS / 32, TAPS = KW * KW;
+    constexpr int OB = ROWS_GROUP, WARPS = THREADS / 32, TAPS = KW * KW;
     constexpr int LEN = segment_len(KW, sizeof(T)), OFF = segment_offset(KW, sizeof(T)), STRIDE = window_stride(KW, sizeof(T));
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geometry& g = a.g;
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(THREADS, 2) morpho_backward_pairs_rows_kernel(
 template <int KW>
 inline size_t pairs_rows_smem(const Geometry& g, int channels)
 {
-    constexpr int OB = 4, WARPS = THREADS / 32, TAPS = KW * KW;
+    constexpr int OB = ROWS_GROUP, WARPS = THREADS / 32, TAPS = KW * KW;
     const size_t o_span = (static_cast<size_t>(channels) + OB - 1) / OB * OB;
     const size_t bytes = (2 * static_cast<size_t>(g.window_elems()) + TAPS * OB + WARPS * TAPS * 32 + o_span * TAPS) * sizeof(float);
     return bytes <= 110 * 1024 ? bytes : 0;

@@ -94,3 +94,32 @@ def test_workload_tap_counts():
     assert WL.taps(8, 64, 64, 512, 512, 11, 11, identity=True) == 16_240_345_088
     assert WL.cfg5_taps(256) == 2_284_570_279_936
     assert M.__version__
+
+
+def test_channel_shares_never_lose_to_one_share(tmp_path):
+    """The rule that divides a tile's output channels among thread blocks (csrc/shares.cuh), on the host: a share that holds
+    part of a group pays for most of the group. Left column: tiles, channels, group, fixed work, `alone`; right: what was measured to be
+    right there (1 = do not divide)."""
+    import os
+    import shutil
+    import subprocess
+    from conftest import ROOT
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    cases = {(104, 4, 4, 2, 0.7): {1}, (104, 4, 1, 5, 0.6): {1}, (592, 4, 4, 2, 0.7): {1}, (1024, 64, 1, 8, 0.6): {1}, (104, 2, 2, 3, 0.6): {1},
+             (20, 12, 4, 2, 0.7): {4, 5, 6}, (120, 12, 4, 2, 0.7): {2}, (120, 10, 4, 2, 0.7): {2}, (104, 12, 4, 2, 0.7): {2, 3, 4},
+             (20, 12, 1, 5, 0.6): {6, 12}, (104, 6, 2, 3, 0.6): {2, 3}, (1, 1, 4, 2, 0.7): {1}}
+    src = tmp_path / "shares.cpp"
+    src.write_text('#include "shares.cuh"\n#include <cstdio>\nint main() {\n'
+                   + "".join(f'    std::printf("%d\\n", mc::channel_shares({t}, {c}, 2, {f}, {g}, {alone}));\n' for t, c, g, f, alone in cases)
+                   + "    for (int count = 1; count < 40; count++) for (int n = 1; n <= count; n++) for (int i = 0; i < n; i++)\n"
+                     "        if (mc::share_begin(count, i, n) >= mc::share_begin(count, i + 1, n)\n"
+                     "            || mc::share_begin(count, i + 1, n) - mc::share_begin(count, i, n) > (count + n - 1) / n) return 1;\n"
+                     "    return mc::share_begin(7, 3, 3) == 7 ? 0 : 1;\n}\n")
+    exe = tmp_path / "shares"
+    subprocess.run([cxx, "-std=c++17", "-D__host__=", "-D__device__=", "-D__forceinline__=inline", "-I", os.path.join(ROOT, "morphocore_b200", "csrc"),
+                    str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
+    for got, (case, right) in zip(map(int, out), cases.items(), strict=True):
+        assert got in right, (case, got)
