@@ -370,7 +370,6 @@ torch::Tensor pair_alphas(const torch::Tensor& alpha, int64_t merge, int64_t out
 struct SmorphCall
 {
     torch::Tensor input4d, weight4d, alphas, output;
-    torch::Tensor raw_weight;   // the structuring element before the re-parametrisation, where the call includes it
 };
 
 /// w~ of the pairs (mc_smorph_reparametrise).
@@ -412,33 +411,42 @@ SmorphCall run_smorph_forward(const torch::Tensor& input, const torch::Tensor& w
     const mc_desc d = make_desc(input4d, call.weight4d, MC_OP_DILATION, merge);
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const TraceRange trace("morphocore::smorph_forward");
-    if (reparametrise)
-    {
-        call.raw_weight = call.weight4d;
-        call.weight4d = reparametrised(d, call.raw_weight, call.alphas, stream);
-    }
+    if (reparametrise) call.weight4d = reparametrised(d, call.weight4d, call.alphas, stream);
     call.output = at::empty({input4d.size(0), call.weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
     check_status(mc_smorph_forward(&d, input4d.data_ptr(), call.weight4d.data_ptr(), call.alphas.data_ptr(), call.output.data_ptr(), stream));
     return call;
 }
 
 /// Gradient of the structuring element as the user holds it, from that of w~; adds to the alpha gradient what flows through
-/// w~ (meaningless where `raw_weight` is not the structuring element, see save_raw_weight).
-torch::Tensor through_reparametrisation(const mc_desc& d, const torch::Tensor& raw_weight, const torch::Tensor& alphas, const torch::Tensor& grad,
-                                        torch::Tensor& grad_alpha_pairs, cudaStream_t stream)
+/// w~. `weight` is the structuring element, undefined where alpha needs no gradient (see save_raw_weight): w~ then stands in for
+/// it, and what it adds to the alpha gradient means nothing.
+/// A backward pass that is itself differentiated (create_graph) takes tensor operations instead of the kernel: the result then
+/// depends on alpha and the structuring element as it does in the reference, where the re-parametrisation is tensor operations
+/// and the operator's own gradients are constants.
+torch::Tensor through_reparametrisation(const mc_desc& d, const torch::Tensor& weight, const torch::Tensor& w_tilde, const torch::Tensor& alpha,
+                                        const torch::Tensor& alphas, const torch::Tensor& grad, torch::Tensor& grad_alpha_pairs, cudaStream_t stream)
 {
+    if (at::GradMode::is_enabled() && weight.defined())
+    {
+        const torch::Tensor t = alpha.numel() == 1 ? torch::tanh(alpha).reshape({1, 1, 1, 1}) : torch::tanh(alpha).reshape({weight.size(0), weight.size(1), 1, 1});
+        const torch::Tensor straight = (1 + t) / 2, mirrored = (1 - t) / 2, flipped = weight.flip({2, 3});
+        const torch::Tensor through_t = mirrored * flipped + straight * weight + t * (weight - flipped) / 2;
+        grad_alpha_pairs = grad_alpha_pairs + ((1 - t * t).reshape({t.size(0), t.size(1)}) * (grad * through_t).sum({2, 3})).view_as(grad_alpha_pairs);
+        return t * (straight * grad + mirrored * grad.flip({2, 3}));
+    }
+    const torch::Tensor raw = weight.defined() ? weight.contiguous() : w_tilde;
     torch::Tensor out = at::empty_like(grad);
-    check_status(mc_smorph_reparametrise_backward(&d, raw_weight.data_ptr(), alphas.data_ptr(), grad.data_ptr(), out.data_ptr(),
-                                                  grad_alpha_pairs.data_ptr(), stream));
+    check_status(mc_smorph_reparametrise_backward(&d, raw.data_ptr(), alphas.data_ptr(), grad.data_ptr(), out.data_ptr(), grad_alpha_pairs.data_ptr(),
+                                                  stream));
     return out;
 }
 
 /// The structuring element before the re-parametrisation is needed by the alpha gradient alone. Where alpha has none it is
-/// not saved, so that a program may change it in place before the backward pass; backward() then hands w~ in its place and
-/// drops the alpha gradient.
-torch::Tensor save_raw_weight(const torch::Tensor& raw_weight, const torch::Tensor& alpha)
+/// not saved, so that a program may change it in place before the backward pass. Otherwise it is saved as the caller's tensor,
+/// through which a differentiated backward pass reaches it.
+torch::Tensor save_raw_weight(bool reparametrise, const torch::Tensor& weight, const torch::Tensor& alpha)
 {
-    return alpha.requires_grad() ? raw_weight : torch::Tensor();
+    return reparametrise && alpha.requires_grad() ? weight : torch::Tensor();
 }
 
 class SmorphFunction : public torch::autograd::Function<SmorphFunction>
@@ -449,7 +457,7 @@ public:
     {
         const SmorphCall call = run_smorph_forward(input, weight, alpha, merge, reparametrise);
         // The backward pass reads the 4-D output: the merge target of MAX and MIN.
-        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d, call.alphas, save_raw_weight(call.raw_weight, alpha)});
+        ctx->save_for_backward({call.output, alpha, call.input4d, call.weight4d, call.alphas, save_raw_weight(reparametrise, weight, alpha)});
         ctx->saved_data["reparametrised"] = reparametrise;
         ctx->saved_data["merge"] = merge;
         ctx->saved_data["input_dims"] = input.dim();
@@ -488,7 +496,7 @@ public:
                                         grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
                                         workspace.defined() ? workspace.data_ptr() : nullptr, ws_bytes, stream));
         if (ctx->saved_data["reparametrised"].toBool())
-            grad_weight = through_reparametrisation(d, raw_weight.defined() ? raw_weight : weight, alphas, grad_weight, grad_alpha_pairs, stream);
+            grad_weight = through_reparametrisation(d, raw_weight, weight, alpha, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph.cpp:96-98).
         torch::Tensor grad_alpha =
@@ -503,7 +511,6 @@ public:
 struct SmorphScmCall
 {
     torch::Tensor input4d, weight4d, alphas, betas, output;
-    torch::Tensor raw_weight;   // as in SmorphCall
 };
 
 SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Tensor& weight, const torch::Tensor& alpha, const torch::Tensor& beta,
@@ -533,11 +540,7 @@ SmorphScmCall run_smorph_scm_forward(const torch::Tensor& input, const torch::Te
     const mc_desc d = make_desc(input4d, call.weight4d, MC_OP_DILATION, MC_MERGE_SMOOTH);
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const TraceRange trace("morphocore::smorph_scm_forward");
-    if (reparametrise)
-    {
-        call.raw_weight = call.weight4d;
-        call.weight4d = reparametrised(d, call.raw_weight, call.alphas, stream);
-    }
+    if (reparametrise) call.weight4d = reparametrised(d, call.weight4d, call.alphas, stream);
     call.output = at::empty({input4d.size(0), call.weight4d.size(0), input4d.size(2), input4d.size(3)}, input4d.options());
     check_status(mc_smorph_scm_forward(&d, input4d.data_ptr(), call.weight4d.data_ptr(), call.alphas.data_ptr(), call.betas.data_ptr(),
                                        call.output.data_ptr(), stream));
@@ -554,7 +557,7 @@ public:
     {
         const SmorphScmCall call = run_smorph_scm_forward(input, weight, alpha, beta, reparametrise);
         // The backward pass reads the 4-D output: the final value of the soft merge.
-        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d, call.alphas, save_raw_weight(call.raw_weight, alpha)});
+        ctx->save_for_backward({call.output, alpha, call.betas, call.input4d, call.weight4d, call.alphas, save_raw_weight(reparametrise, weight, alpha)});
         ctx->saved_data["reparametrised"] = reparametrise;
         ctx->saved_data["input_dims"] = input.dim();
         ctx->saved_data["weight_dims"] = weight.dim();
@@ -591,7 +594,7 @@ public:
                                             grad_output.data_ptr(), grad_input.data_ptr(), grad_weight.data_ptr(), grad_alpha_pairs.data_ptr(),
                                             grad_beta.data_ptr(), workspace.data_ptr(), ws_bytes, stream));
         if (ctx->saved_data["reparametrised"].toBool())
-            grad_weight = through_reparametrisation(d, raw_weight.defined() ? raw_weight : weight, alphas, grad_weight, grad_alpha_pairs, stream);
+            grad_weight = through_reparametrisation(d, raw_weight, weight, alpha, alphas, grad_weight, grad_alpha_pairs, stream);
 
         // A single alpha shared by every pair receives the gradient of all of them (csrc/cpp/smorph_scm.cpp:81-83).
         torch::Tensor grad_alpha =

@@ -401,6 +401,37 @@ def test_smorph_reparametrisation_kernel(F, shape, k):
         assert torch.equal(F.smorph(x, w, a, beta, merge), y)
 
 
+@pytest.mark.parametrize("shape", ["pairs", "single", "identity", "identity_1d", "smooth", "strided"])
+def test_smorph_gradients_keep_their_graph_through_the_reparametrisation(F, shape):
+    """create_graph: the gradients of functional.smorph depend on alpha and the structuring element through the
+    re-parametrisation, as in the chain of tensor operations (the operator's own gradients are constants in both). First and
+    second gradients in double against that chain: same operations, sums of k terms."""
+    torch.manual_seed(8)
+    c, identity = 4, shape.startswith("identity")
+    leaf = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda").requires_grad_(True)   # noqa: E731
+    x, w = leaf(2, c, 13, 18), leaf(c if identity else 3, 1 if identity else c, 5, 3)
+    a = leaf(1) if shape == "single" else leaf(c) if shape == "identity_1d" else leaf(c, 1) if identity else leaf(3, c)
+    held = leaf(3, 5, c, 3).transpose(1, 2) if shape == "strided" else w     # a structuring element that is not contiguous
+    beta = leaf(3) if shape == "smooth" else None
+    gy = torch.randn(2, w.shape[0], 13, 18, dtype=torch.float64, device="cuda")
+    cw, ca = torch.randn_like(w), torch.randn_like(a)
+    merge = "identity" if identity else "sum"
+
+    def chain():
+        t = torch.tanh(a)
+        t = t.view(-1, 1, 1, 1) if identity or a.dim() == 1 else t[..., None, None]
+        tilde = t * ((1 - t) / 2 * held.flip((-2, -1)) + (1 + t) / 2 * held)
+        ops = torch.ops.morphocore
+        return ops.smorph(x, tilde, a, 5 if identity else 2) if beta is None else ops.smorph_scm(x, tilde, a, beta)
+
+    def derivatives(y):
+        gw, ga = torch.autograd.grad(y, (held, a), gy, create_graph=True)
+        return (gw, ga) + torch.autograd.grad((gw * cw).sum() + (ga * ca).sum(), (held, a))
+
+    for p, q in zip(derivatives(F.smorph(x, held, a, beta, merge)), derivatives(chain())):
+        assert p.shape == q.shape and (p - q).abs().max() <= 1e-11 * q.abs().max().clamp_min(1.0)
+
+
 def test_parameters_may_change_in_place_before_the_backward_pass(F):
     """Erosion differentiates with the structuring element of the call, and so does smorph where alpha has no gradient (with
     one, autograd refuses the call): changing the parameter in place between the two passes is allowed and changes nothing."""
