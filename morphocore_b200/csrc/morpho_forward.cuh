@@ -283,8 +283,8 @@ __device__ __forceinline__ void window_extremum(T (&acc)[OB][PATCH_H][PATCH_W], 
 /// The same for a 3 x 3 structuring element in float and an even number of output channels, finished pixel by pixel: the
 /// thread's 4 x 6 window elements stay in registers, doubled for the packed adds, and the nine candidates of a pixel meet the
 /// initial value in four three-input extrema and one two-input one (row by row it takes six instructions); `emit(o, rr, j,
-/// value)` merges each result at once, so no array of running extrema is held. (16, 32, 56, 56) -> 64 channels: 154 -> 103 us
-/// together with the staging below.
+/// value)` merges each result at once, so no array of running extrema is held. (16, 32, 56, 56) -> 64 channels: 154 -> 113 us
+/// together with the staging below (erosion, mean; dilation, sum: 150 -> 109).
 template <bool IS_MIN, int OB, typename Emit>
 __device__ __forceinline__ void window_extremum_3x3(const float* __restrict__ win, const float* __restrict__ wk, int o_count, int tx, int ty, Emit emit)
 {
